@@ -1,0 +1,57 @@
+// Instantiations and launches of the CG with the matrix on chip
+// (ks_chip_cg.cuh).
+#include "ks_chip_cg.cuh"
+
+namespace ks {
+
+template <class VT, int NDG, int RJ, bool kTile>
+static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  auto fn = k_cg_chip<VT, NDG, RJ, kTile>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  if (e != cudaSuccess) return e;
+  if (probe) {
+    int b = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kChipThreads, sh.smem);
+    *fits = e == cudaSuccess && b >= 1;
+    return e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sh.G);
+  cfg.blockDim = dim3(kChipThreads);
+  cfg.dynamicSmemBytes = sh.smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ctx->launches++;
+  ProfLaunch pl(ctx, cls);
+  return cudaLaunchKernelEx(&cfg, fn, a);
+}
+
+template <class VT, int NDG, bool kTile>
+static cudaError_t chip_launch_d(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  if (sh.rj == 1) return chip_launch_n<VT, NDG, 1, kTile>(ctx, a, sh, probe, fits, cls);
+  if (sh.rj == 2) return chip_launch_n<VT, NDG, 2, kTile>(ctx, a, sh, probe, fits, cls);
+  if (sh.rj == 4) return chip_launch_n<VT, NDG, 4, kTile>(ctx, a, sh, probe, fits, cls);
+  if (sh.rj == 8) return chip_launch_n<VT, NDG, 8, kTile>(ctx, a, sh, probe, fits, cls);
+  if constexpr (sizeof(VT) == 4) return chip_launch_n<VT, NDG, 16, kTile>(ctx, a, sh, probe, fits, cls);
+  return cudaErrorInvalidValue;
+}
+template <class VT>
+static cudaError_t chip_launch_t(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  if (sh.tile) return chip_launch_d<VT, 7, true>(ctx, a, sh, probe, fits, cls);
+  if (a.nd == 7) return chip_launch_d<VT, 7, false>(ctx, a, sh, probe, fits, cls);
+  if (a.nd == 5) return chip_launch_d<VT, 5, false>(ctx, a, sh, probe, fits, cls);
+  return chip_launch_d<VT, 0, false>(ctx, a, sh, probe, fits, cls);
+}
+
+cudaError_t chip_launch_f64(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  return chip_launch_t<double>(ctx, a, sh, probe, fits, cls);
+}
+cudaError_t chip_launch_f32(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  return chip_launch_t<float>(ctx, a, sh, probe, fits, cls);
+}
+
+}  // namespace ks

@@ -103,6 +103,9 @@ struct CsrDev {
   // for i < o lands in the zero pad. dia_sym = 0: all dia_nd diagonals, each
   // of n elements (dia_ds = n, dia_pad = 0).
   int dia_sym = 0;
+  // 1: a 7-point stencil on a box of lines of dia_off[5] rows and planes of
+  // dia_off[6] rows, without an entry across the end of a line or plane.
+  int dia_box = 0;
   int dia_pad = 0;
   long long dia_ds = 0;
 };

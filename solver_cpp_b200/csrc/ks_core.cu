@@ -347,8 +347,25 @@ static void free_dia(CsrDev &A) {
   A.dia_mask = nullptr;
   A.dia_nd = 0;
   A.dia_sym = 0;
+  A.dia_box = 0;
   A.dia_pad = 0;
   A.dia_ds = 0;
+}
+
+// Sets *bad if a row at the end of a line (b rows) or of a plane (c rows) has
+// an entry on the diagonal that leaves it: mask bits 0..6 are the diagonals
+// -c, -b, -1, 0, 1, b, c.
+__global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, int b, int c, int *bad) {
+  const int ny = c / b;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int x = i % b, y = (i / b) % ny;
+    unsigned out = 0;
+    if (x == 0) out |= 1u << 2;
+    if (x == b - 1) out |= 1u << 4;
+    if (y == 0) out |= 1u << 1;
+    if (y == ny - 1) out |= 1u << 5;
+    if (mask[i] & out) *bad = 1;
+  }
 }
 
 // Builds the diagonal copy when the matrix qualifies (CsrDev::dia_*); leaves
@@ -420,6 +437,27 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
     }
     sym = flag == 0;
   }
+  // A 7-point stencil on a box: diagonals 0, +-1, +-b, +-c with c a multiple of
+  // b and n one of c, and no entry that reaches across the end of a line or
+  // of a plane
+  bool box = o.nd == 7 && cmin == 0 && cmax == A.n && o.off[3] == 0 && o.off[4] == 1 && o.off[5] > 1 &&
+             o.off[6] > o.off[5] && o.off[6] % o.off[5] == 0 && A.n % o.off[6] == 0;
+  for (int k = 0; box && k < 3; k++) box = o.off[k] == -o.off[6 - k];
+  if (box) {
+    int flag = 0;
+    e = cudaMemsetAsync(d_buf, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess) {
+      k_dia_boxcheck<<<g, 256, 0, ctx->stream>>>(A.dia_mask, A.n, o.off[5], o.off[6], d_buf);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, d_buf, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) {
+      cudaFree(d_buf);
+      return cuda_fail(ctx, e, "box check");
+    }
+    box = flag == 0;
+  }
   cudaFree(d_buf);
   long long ds = A.n, stored = len + 8;
   int pad = 0;
@@ -458,6 +496,7 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   A.dia_cmin = (int)cmin;
   A.dia_cmax = (int)cmax;
   A.dia_sym = sym ? 1 : 0;
+  A.dia_box = box ? 1 : 0;
   A.dia_pad = pad;
   A.dia_ds = ds;
   return KS_OK;
@@ -697,8 +736,8 @@ ks_status ks_ctx_create(int device, ks_ctx **out) {
     return fail(KS_OUT_OF_MEMORY);
   std::memset(ctx->h_snap, 0, sizeof(int) * ctx->nflags);
   if (cudaMalloc(&ctx->d_stage, sizeof(double) * kStageLen) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
-  // barrier state of the on-chip inner CG: 32 bytes + one flag per SM
-  if (cudaMalloc(&ctx->ir_sync, 64 + 8 * (size_t)ctx->num_sms) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
+  // barrier state of the on-chip kernels (ir_sync_bytes of one CTA per SM)
+  if (cudaMalloc(&ctx->ir_sync, 64 + 40 * (size_t)ctx->num_sms) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
   ctx->flag_events = new cudaEvent_t[ctx->nflags];
   for (int i = 0; i < ctx->nflags; i++) {
     if (cudaEventCreateWithFlags(&ctx->flag_events[i], cudaEventDisableTiming) != cudaSuccess)

@@ -51,22 +51,27 @@ namespace ks {
 constexpr int kIrThreads = 1024;  // threads per CTA, one CTA per SM
 constexpr int kIrMaxK = 32;       // rows per thread (r and q in 64 TMEM columns)
 constexpr int kIrWarps = kIrThreads / 32;
+constexpr int kIrMaxGrid = 256;  // CTAs a reduction takes (one per SM)
+constexpr int kIrMaxSums = 2;    // values one reduction carries
 
 // Barrier state in device memory, zeroed before every launch: the grid
-// reductions' counter, generation and result, then one publication flag per
-// CTA (ir_sync_bytes).
+// reductions' arrival counter, one publication flag per CTA, then the tagged
+// slots of k_cg_chip's reductions (two per CTA, ks_chip_cg.cuh).
 struct IrSync {
   unsigned long long count;  // CTA arrivals at the reductions, all generations
   unsigned long long reserved;
 };
-static_assert(sizeof(IrSync) % 8 == 0, "the publication flags follow IrSync");
+static_assert(sizeof(IrSync) == 16, "the flags and the 16-byte slots follow IrSync");
 
 // Flag of CTA q right after IrSync: the last generation of p it has published.
 __device__ __forceinline__ unsigned long long *ir_pub(IrSync *s, int q) {
   return reinterpret_cast<unsigned long long *>(s + 1) + q;
 }
 
-inline size_t ir_sync_bytes(int G) { return sizeof(IrSync) + sizeof(unsigned long long) * (size_t)G; }
+inline size_t ir_sync_bytes(int G) {
+  return sizeof(IrSync) + sizeof(unsigned long long) * (size_t)((G + 1) & ~1) +
+         sizeof(ulonglong2) * 2 * (size_t)G;
+}
 
 struct IrArgs {
   const void *rin;  // inner solve: r rounded to FP32; whole solve: b (FP64); n entries
@@ -160,8 +165,6 @@ __device__ __forceinline__ void ir_block_sum(double (&v)[N], double (*sh)[kIrWar
 // have, then sums all partials itself, every load issued before the first
 // add and the terms added in one fixed order, so every CTA obtains the same
 // bits. Returns false when a wait ran out (the timeout flag is then set).
-constexpr int kIrMaxGrid = 256;  // CTAs a reduction takes (one per SM)
-constexpr int kIrMaxSums = 2;    // values one reduction carries
 
 // A grid reduction in two halves, so that work which does not need the sums
 // runs while the other CTAs arrive: ir_red_post adds the CTA's values (a
@@ -1599,7 +1602,7 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_cr_onchip(DiaT<double> D, IrA
 // lines stay cached), p 128-byte aligned: after the on-chip kernels' evict_last
 // loads, so that the diagonal copy does not keep its place in L2 ahead of
 // later work.
-__global__ void k_l2_normal(const char *p, unsigned long long bytes) {
+static __global__ void k_l2_normal(const char *p, unsigned long long bytes) {
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x * 128ull;
   for (unsigned long long o = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) * 128ull; o < bytes;
        o += stride)

@@ -18,6 +18,7 @@
 #include "ks_ops.cuh"
 #include "ks_state.cuh"
 #include "ks_resident.cuh"
+#include "ks_chip_cg.cuh"
 #include "ks_inner_resident.cuh"
 
 namespace ks {
@@ -799,6 +800,38 @@ inline bool run_cg_resident(const Env<double> &E, const double *b, double *x, ks
   return true;
 }
 
+// From this size on the matrix-on-chip kernel is the faster one (us per
+// iteration, cluster / on chip: 64^2 2.70 / 3.20, 20^3 3.62 / 3.67, 96^2 4.43 /
+// 3.34, 24^3 5.40 / 3.59, 181^2 6.67 / 3.57, 31^3 8.50 / 4.68).
+constexpr long long kChipMinRows = 8192;
+
+// Larger systems whose matrix fits on chip across the GPU as well as their
+// vectors (up to about 4,096 rows per SM in FP64, one GPU, a diagonal copy;
+// ks_params.cluster_solve 0): the whole solve as one cooperative kernel
+// (k_cg_chip, ks_chip_cg.cuh). Returns false, having launched nothing, when
+// the system does not qualify.
+inline bool run_cg_chip(const Env<double> &E, const double *b, double *x, double *R, ks_status *s) {
+  if (E.sp.cluster_solve || !E.outer || E.comm || E.mvals != KS_FP64 || !E.A->dia_nd || !E.A->dia_val) return false;
+  ks_ctx *ctx = E.ctx;
+  ChipShape sh;
+  // R takes the first two workspace slots
+  if (!chip_shape<double>(ctx, *E.A, E.n, &sh) || reinterpret_cast<uintptr_t>(R) % 16) return false;
+  const IrArgs ir{b, x, R, E.st, nullptr, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns, (int)E.n, sh.rpc, sh.rj, 1, 0};
+  const ChipArgs a = chip_args<double, double>(*E.A, ir, sh, 0);
+  bool fits = false;
+  if (chip_launch<double>(ctx, a, sh, true, &fits, 0) != cudaSuccess || !fits) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  launch_scalar(ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
+  cudaError_t e = cudaMemsetAsync(ctx->ir_sync, 0, ir_sync_bytes(sh.G), ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(R, 0, chip_r_bytes<double>(E.n), ctx->stream);
+  // a profiled solve counts the whole solve as one SpMV-class launch
+  if (e == cudaSuccess) e = chip_launch<double>(ctx, a, sh, false, &fits, kMv);
+  *s = e == cudaSuccess ? KS_OK : cuda_fail(ctx, e, "on-chip CG launch");
+  return true;
+}
+
 // Larger systems whose vectors fit on chip across the GPU (up to about 14,400
 // rows per SM in FP64, one GPU, a diagonal copy; ks_params.cluster_solve 0):
 // the whole solve as one cooperative kernel of one CTA per SM, r and q in
@@ -839,6 +872,7 @@ template <class VT>
 ks_status run_cg(const Env<VT> &E, const VT *b, VT *x, VT *ws, double *dws) {
   if constexpr (std::is_same<VT, double>::value) {
     ks_status s = KS_OK;
+    if (E.n > kChipMinRows && run_cg_chip(E, b, x, ws, &s)) return s;
     if (run_cg_resident(E, b, x, &s)) return s;
     if (run_cg_onchip(E, b, x, ws, &s)) return s;
   }
@@ -2310,20 +2344,6 @@ struct InnerResBufs {
   int stencil;  // P zero-padded for the stencil path (ir_stencil_ok)
 };
 
-// One inner solve with the on-chip kernel (its start already issued).
-inline ks_status run_cg_inner_resident(const Env<float> &E, const InnerResBufs &B, const IrShape &sh) {
-  ks_ctx *ctx = E.ctx;
-  IrArgs a{B.r, B.x, B.P, E.st, E.outer_done, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns,
-           (int)E.n, sh.rpc, sh.K, 0, B.stencil};
-  cudaError_t e = cudaMemsetAsync(ctx->ir_sync, 0, ir_sync_bytes(sh.G), ctx->stream);
-  if (e == cudaSuccess) {
-    bool fits = false;
-    e = E.mvals == KS_BF16 ? ir_launch<float, __nv_bfloat16>(ctx, *E.A, a, sh, false, &fits, kMvLow)
-                           : ir_launch<float, float>(ctx, *E.A, a, sh, false, &fits, kMvLow);
-  }
-  return e == cudaSuccess ? KS_OK : cuda_fail(ctx, e, "on-chip inner CG launch");
-}
-
 template <class VT>
 struct InnerRunner {
   // Outer-precision view (VT) and the inner environment.
@@ -2343,9 +2363,41 @@ struct InnerRunner {
   bool res_cg = false;
   InnerResBufs fb{};
   IrShape sh{};
+  bool chip = false;  // the matrix on chip too (k_cg_chip)
+  ChipShape csh{};
+  unsigned long long tag = 0;  // the last tag used on fb.P
+  ChipArgs chip_args(const IrArgs &a) const {
+    return iprec == KS_BF16 ? ks::chip_args<float, __nv_bfloat16>(*E32.A, a, csh, tag)
+                            : ks::chip_args<float, float>(*E32.A, a, csh, tag);
+  }
   void setup_resident();
   void solve(const VT *b, VT *z);
 };
+
+// One inner solve with the on-chip kernel (its start already issued).
+inline ks_status run_cg_inner_resident(InnerRunner<double> &I) {
+  const Env<float> &E = I.E32;
+  const InnerResBufs &B = I.fb;
+  ks_ctx *ctx = E.ctx;
+  IrArgs a{B.r, B.x, B.P, E.st, E.outer_done, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns,
+           (int)E.n, I.sh.rpc, I.sh.K, 0, B.stencil};
+  cudaError_t e = cudaMemsetAsync(ctx->ir_sync, 0, ir_sync_bytes(I.chip ? I.csh.G : I.sh.G), ctx->stream);
+  if (e == cudaSuccess) {
+    bool fits = false;
+    if (I.chip) {
+      // the tags of this launch follow the last one's; FP32 keeps 32 bits of them
+      if (I.tag + (unsigned long long)E.sp.maxloop + 2 > 0xffffffffull) {
+        e = cudaMemsetAsync(B.P, 0, chip_r_bytes<float>(E.n), ctx->stream);
+        I.tag = 0;
+      }
+      if (e == cudaSuccess) e = chip_launch<float>(ctx, I.chip_args(a), I.csh, false, &fits, kMvLow);
+      I.tag += (unsigned long long)E.sp.maxloop + 1;
+    } else
+      e = E.mvals == KS_BF16 ? ir_launch<float, __nv_bfloat16>(ctx, *E.A, a, I.sh, false, &fits, kMvLow)
+                             : ir_launch<float, float>(ctx, *E.A, a, I.sh, false, &fits, kMvLow);
+  }
+  return e == cudaSuccess ? KS_OK : cuda_fail(ctx, e, "on-chip inner CG launch");
+}
 
 // The on-chip inner CG applies where the inner method is CG in FP32 or with
 // BF16 values, on one GPU, the SpMV reads a diagonal copy of those values,
@@ -2356,8 +2408,21 @@ void InnerRunner<VT>::setup_resident() {
   if (method != KS_CG || iprec == KS_FP64 || E32.comm || !E32.A || !E32.A->dia_nd) return;
   if (iprec == KS_FP32 ? !E32.A->dia_val32 : !E32.A->dia_val16) return;
   if (vec_count(KS_CG, E32.sp, E32.n, sizeof(float), ctx->l2_bytes) < 3) return;  // P (two slots) and r
-  if (!ir_shape<float>(ctx, E32.n, &sh)) return;
   bool fits = false;
+  if (E32.sp.maxloop < (1ll << 31) && chip_shape<float>(ctx, *E32.A, E32.n, &csh) &&
+      reinterpret_cast<uintptr_t>(Ws<float>{ws32, E32.ld, E32.off}.take()) % 8 == 0 && chip_launch<float>(ctx, chip_args(IrArgs{}), csh, true, &fits, 0) == cudaSuccess && fits) {
+    Ws<float> W{ws32, E32.ld, E32.off};
+    fb.P = W.take(2);
+    fb.r = W.take();
+    fb.x = z32;
+    if (cudaMemsetAsync(fb.P, 0, chip_r_bytes<float>(E32.n), ctx->stream) == cudaSuccess) {
+      res_cg = chip = true;
+      return;
+    }
+  }
+  (void)cudaGetLastError();
+  fits = false;
+  if (!ir_shape<float>(ctx, E32.n, &sh)) return;
   const IrArgs none{};
   const cudaError_t e = iprec == KS_BF16 ? ir_launch<float, __nv_bfloat16>(ctx, *E32.A, none, sh, true, &fits, 0)
                                          : ir_launch<float, float>(ctx, *E32.A, none, sh, true, &fits, 0);
@@ -2393,7 +2458,7 @@ void InnerRunner<VT>::solve(const VT *b, VT *z) {
     } else if (res_cg) {
       const Stop os{nullptr, E32.outer_done};
       launch_vec(ctx, n, CgInStartOp<float>{b, fb.r, E32.st, E32.sp.eps, E32.sp.maxloop}, os);
-      status = run_cg_inner_resident(E32, fb, sh);
+      status = run_cg_inner_resident(*this);
       launch_vec(ctx, n, CgInFinalOp<float>{fb.x, E32.st, z, nullptr, nullptr, 0}, os);
     } else {
       launch_vec(ctx, n, ConvertOp<double, float>{b, b32}, Stop{nullptr, E32.outer_done});
@@ -2454,7 +2519,7 @@ ks_status run_vpcg(const Env<VT> &E, const VT *b, VT *x, VT *ws, double *dws, In
         const Stop os{nullptr, F.outer_done};
         I.calls++;
         launch_vec(E.ctx, E.n, CgInStartOp<float>{r, I.fb.r, F.st, F.sp.eps, F.sp.maxloop}, os);
-        if (I.status == KS_OK) I.status = run_cg_inner_resident(F, I.fb, I.sh);
+        if (I.status == KS_OK) I.status = run_cg_inner_resident(I);
         launch_vec(E.ctx, E.n, CgInFinalOp<float>{I.fb.x, F.st, z, r, E.st, 1}, os);
         Lr = 1;
         vec(E, CopyOp<VT>{z, R.slot(Lr)});
@@ -2480,7 +2545,7 @@ ks_status run_vpcg(const Env<VT> &E, const VT *b, VT *x, VT *ws, double *dws, In
         } else {
           vec(E, VpXrStartOp<float>{x, r, p, mvv, E.st, I.fb.r, F.st, F.sp.eps, F.sp.maxloop});
         }
-        if (I.status == KS_OK) I.status = run_cg_inner_resident(F, I.fb, I.sh);
+        if (I.status == KS_OK) I.status = run_cg_inner_resident(I);
         launch_vec(E.ctx, E.n, CgInFinalOp<float>{I.fb.x, F.st, nullptr, r, E.st, 2},
                    Stop{nullptr, F.outer_done});
         VT *pn = defer ? R.slot(Lr + 1) : p;
