@@ -108,6 +108,9 @@ struct CsrDev {
   int dia_box = 0;
   int dia_pad = 0;
   long long dia_ds = 0;
+  // 1: the entries of each diagonal are all one value, dia_cv[d], bit for bit.
+  int dia_cst = 0;
+  double dia_cv[kMaxDiag] = {};
 };
 
 template <class MT>

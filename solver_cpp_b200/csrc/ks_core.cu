@@ -348,6 +348,7 @@ static void free_dia(CsrDev &A) {
   A.dia_nd = 0;
   A.dia_sym = 0;
   A.dia_box = 0;
+  A.dia_cst = 0;
   A.dia_pad = 0;
   A.dia_ds = 0;
 }
@@ -355,7 +356,11 @@ static void free_dia(CsrDev &A) {
 // Sets *bad if a row at the end of a line (b rows) or of a plane (c rows) has
 // an entry on the diagonal that leaves it: mask bits 0..6 are the diagonals
 // -c, -b, -1, 0, 1, b, c.
-__global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, int b, int c, int *bad) {
+struct DiagFacts {
+  unsigned long long lo[kMaxDiag], hi[kMaxDiag];  // least and greatest bit pattern of each diagonal's entries
+  int bad;  // entries across the end of a line or plane
+};
+__global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, int b, int c, DiagFacts *f) {
   const int ny = c / b;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int x = i % b, y = (i / b) % ny;
@@ -364,7 +369,42 @@ __global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, in
     if (x == b - 1) out |= 1u << 4;
     if (y == 0) out |= 1u << 1;
     if (y == ny - 1) out |= 1u << 5;
-    if (mask[i] & out) *bad = 1;
+    if (mask[i] & out) f->bad = 1;
+  }
+}
+
+// The least and greatest bit pattern of every diagonal's entries.
+__global__ void k_dia_range(const double *__restrict__ dval, const unsigned char *__restrict__ mask, int n, int nd,
+                            DiagFacts *f) {
+  unsigned long long lo[kMaxDiag], hi[kMaxDiag];
+#pragma unroll
+  for (int d = 0; d < kMaxDiag; d++) {
+    lo[d] = ~0ull;
+    hi[d] = 0;
+  }
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n;
+       r += (long long)gridDim.x * blockDim.x) {
+    const unsigned m = mask[r];
+#pragma unroll
+    for (int d = 0; d < kMaxDiag; d++) {
+      if (d < nd && ((m >> d) & 1u)) {
+        const unsigned long long u = (unsigned long long)__double_as_longlong(dval[(long long)d * n + r]);
+        lo[d] = min(lo[d], u);
+        hi[d] = max(hi[d], u);
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < kMaxDiag; d++) {
+    if (d >= nd) break;
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(&f->lo[d], lo[d]);
+      atomicMax(&f->hi[d], hi[d]);
+    }
   }
 }
 
@@ -439,25 +479,30 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   }
   // A 7-point stencil on a box: diagonals 0, +-1, +-b, +-c with c a multiple of
   // b and n one of c, and no entry that reaches across the end of a line or
-  // of a plane
+  // of a plane. And whether each diagonal's entries are all one value.
   bool box = o.nd == 7 && cmin == 0 && cmax == A.n && o.off[3] == 0 && o.off[4] == 1 && o.off[5] > 1 &&
              o.off[6] > o.off[5] && o.off[6] % o.off[5] == 0 && A.n % o.off[6] == 0;
   for (int k = 0; box && k < 3; k++) box = o.off[k] == -o.off[6 - k];
-  if (box) {
-    int flag = 0;
-    e = cudaMemsetAsync(d_buf, 0, sizeof(int), ctx->stream);
-    if (e == cudaSuccess) {
-      k_dia_boxcheck<<<g, 256, 0, ctx->stream>>>(A.dia_mask, A.n, o.off[5], o.off[6], d_buf);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, d_buf, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) {
-      cudaFree(d_buf);
-      return cuda_fail(ctx, e, "box check");
-    }
-    box = flag == 0;
+  DiagFacts f{};
+  DiagFacts *d_f = nullptr;
+  e = cudaMalloc(&d_f, sizeof(f));
+  for (int k = 0; k < kMaxDiag; k++) f.lo[k] = ~0ull;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_f, &f, sizeof(f), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) {
+    if (box) k_dia_boxcheck<<<g, 256, 0, ctx->stream>>>(A.dia_mask, A.n, o.off[5], o.off[6], d_f);
+    k_dia_range<<<g, 256, 0, ctx->stream>>>(A.dia_val, A.dia_mask, A.n, o.nd, d_f);
+    e = cudaGetLastError();
   }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&f, d_f, sizeof(f), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  cudaFree(d_f);
+  if (e != cudaSuccess) {
+    cudaFree(d_buf);
+    return cuda_fail(ctx, e, "diagonal facts");
+  }
+  box = box && f.bad == 0;
+  bool cst = true;
+  for (int k = 0; k < o.nd; k++) cst = cst && f.lo[k] == f.hi[k];
   cudaFree(d_buf);
   long long ds = A.n, stored = len + 8;
   int pad = 0;
@@ -497,6 +542,11 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   A.dia_cmax = (int)cmax;
   A.dia_sym = sym ? 1 : 0;
   A.dia_box = box ? 1 : 0;
+  A.dia_cst = cst ? 1 : 0;
+  for (int k = 0; k < kMaxDiag; k++) {
+    A.dia_cv[k] = 0.0;
+    if (cst && k < o.nd) std::memcpy(&A.dia_cv[k], &f.lo[k], sizeof(double));
+  }
   A.dia_pad = pad;
   A.dia_ds = ds;
   return KS_OK;

@@ -582,6 +582,18 @@ __device__ __forceinline__ void ir_p4(const VT *sp, const VT *P, int r0, int nr,
   }
 }
 
+// kC: every diagonal's entries are one value (DiaT::cst): the values come from
+// the kernel's parameters and nothing is read. A template parameter of the
+// kernels: chosen at run time inside them, the two ways spill registers.
+template <bool kC, class MT>
+__device__ __forceinline__ bool ir_const(const DiaT<MT> &D, int d, IrVals<MT> &v) {
+  if constexpr (kC) {
+#pragma unroll
+    for (int e = 0; e < kIrQ; e++) v.v[e] = D.cv[d];
+  }
+  return kC;
+}
+
 // q = A p for the 4 consecutive rows i0 .. i0+3 (local li0 .. li0+3, i0 a
 // multiple of 4) of a thread, diagonals in ascending offset order (the
 // row's CSR order), in batches whose loads are all issued before the batch
@@ -589,7 +601,7 @@ __device__ __forceinline__ void ir_p4(const VT *sp, const VT *P, int r0, int nr,
 // two aligned quads around it and a funnel by o mod 4 (uniform across the
 // warp). Every diagonal's value is loaded (zeros where a row has none); FP64
 // adds only the terms the row's mask names, FP32 adds every one.
-template <class VT, class MT, int NDG>
+template <class VT, class MT, int NDG, bool kC>
 __device__ __forceinline__ void ir_quad_mv(const DiaT<MT> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
                                            int nd, VT (&q)[kIrQ]) {
   constexpr int KD = NDG > 0 ? NDG : kMaxDiag;
@@ -615,7 +627,8 @@ __device__ __forceinline__ void ir_quad_mv(const DiaT<MT> &D, const VT *P, const
 #pragma unroll
     for (int u = 0; u < B; u++) {
       const int d = d0 + u;
-      if (d < KD && (NDG > 0 || d < nd)) ir_vals<MT>(D.vb[d] + (i0 + D.vs[d]), full, li0, nr, av[u]);
+      if (d < KD && (NDG > 0 || d < nd) && !ir_const<kC>(D, d, av[u]))
+        ir_vals<MT>(D.vb[d] + (i0 + D.vs[d]), full, li0, nr, av[u]);
     }
 #pragma unroll
     for (int u = 0; u < B; u++) {
@@ -684,7 +697,7 @@ __device__ __forceinline__ VT ir_val(const IrVals<MT> &a, int e) {
 // (ir_quad_mv reads a clamped column instead): the term adds a zero to a sum
 // that starts at +0, which leaves it unchanged, so the terms and their order
 // are ir_quad_mv's and so are the results.
-template <class VT, class MT, int NDG>
+template <class VT, class MT, int NDG, bool kC>
 __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
                                               const VT (&pv)[kIrQ], VT (&q)[kIrQ]) {
   static_assert(NDG == 5 || NDG == 7, "stencil path: 5 or 7 diagonals");
@@ -698,9 +711,11 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
   const VT pm1 = li0 >= 1 ? sp[li0 - 1] : __ldcg(P + (i0 - 1));
   const VT pp4 = li0 + kIrQ < nr ? sp[li0 + kIrQ] : __ldcg(P + (i0 + kIrQ));
   IrVals<MT> vm1, v1;
-  ir_vals4<MT>(D.vb[H + 1] + i0, v1);
+  if (!ir_const<kC>(D, H + 1, v1)) ir_vals4<MT>(D.vb[H + 1] + i0, v1);
   MT m1s = (MT)0;
-  if (sym)
+  if (ir_const<kC>(D, H - 1, vm1))
+    m1s = D.cv[H - 1];
+  else if (sym)
     m1s = ir_ld<MT>(D.vb[H + 1] + (i0 - 1));
   else
     ir_vals4<MT>(D.vb[H - 1] + i0, vm1);
@@ -719,7 +734,7 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
   auto far = [&](int k) {
     const int off = D.off[k];
     IrVals<MT> av;
-    ir_vals4<MT>(D.vb[k] + (i0 + D.vs[k]), av);
+    if (!ir_const<kC>(D, k, av)) ir_vals4<MT>(D.vb[k] + (i0 + D.vs[k]), av);
     VT p[kIrQ], val[kIrQ];
     const int lc = li0 + off;
     if (lc >= 0 && lc + kIrQ <= nr)
@@ -748,7 +763,7 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
   }
   {
     IrVals<MT> v0;
-    ir_vals4<MT>(D.vb[H] + i0, v0);
+    if (!ir_const<kC>(D, H, v0)) ir_vals4<MT>(D.vb[H] + i0, v0);
     VT val[kIrQ];
 #pragma unroll
     for (int e = 0; e < kIrQ; e++) val[e] = ir_val<VT, MT>(v0, e);
@@ -767,7 +782,7 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
 
 // The solve (see the top of this file). Returns the stopping code, or -1
 // when a wait ran out; *xw: x was written (one update at least).
-template <class VT, class MT, int NDG>
+template <class VT, class MT, int NDG, bool kC>
 __device__ __forceinline__ int ir_body(const DiaT<MT> &D, const IrArgs &a, VT *sp, VT *sx, uint32_t tm,
                                        long long *Lout, double *alpha_out, double *beta_out, double *rr_out,
                                        bool *xw) {
@@ -862,11 +877,11 @@ __device__ __forceinline__ int ir_body(const DiaT<MT> &D, const IrArgs &a, VT *s
       bool st_done = false;
       if constexpr (NDG == 5 || NDG == 7) {
         if (a.stencil && li0 + kIrQ <= nr) {
-          ir_quad_mv_st<VT, MT, NDG>(D, P, sp, r0, nr, li0, pv, q);
+          ir_quad_mv_st<VT, MT, NDG, kC>(D, P, sp, r0, nr, li0, pv, q);
           st_done = true;
         }
       }
-      if (!st_done) ir_quad_mv<VT, MT, NDG>(D, P, sp, r0, nr, li0, nd, q);
+      if (!st_done) ir_quad_mv<VT, MT, NDG, kC>(D, P, sp, r0, nr, li0, nd, q);
 #pragma unroll
       for (int e = 0; e < kIrQ; e++)
         if (li0 + e < nr) acc = add_rn(acc, mul_rn(widen(pv[e]), widen(q[e])));
@@ -983,7 +998,7 @@ __device__ __forceinline__ int ir_body(const DiaT<MT> &D, const IrArgs &a, VT *s
   return code;
 }
 
-template <class VT, class MT, int NDG>
+template <class VT, class MT, int NDG, bool kC = false>
 __global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaT<MT> D, IrArgs a) {
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
   __shared__ uint32_t s_tmem;
@@ -1007,7 +1022,7 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaT<MT> D, IrArgs 
   long long L = 0;
   double alpha = 0.0, beta = 0.0, rr = 0.0;
   bool xw = false;
-  const int code = ir_body<VT, MT, NDG>(D, a, sp, sx, tm, &L, &alpha, &beta, &rr, &xw);
+  const int code = ir_body<VT, MT, NDG, kC>(D, a, sp, sx, tm, &L, &alpha, &beta, &rr, &xw);
   if (code >= 0) {
     // x out (a whole solve writes its zeros too): thread t reads rows other
     // threads updated last (the loop may end right after an update pass), so
@@ -1064,7 +1079,7 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaT<MT> D, IrArgs 
 // index order). Every wait is bounded (ir_allreduce, ir_publish_sync).
 constexpr int kIbVecs = 6;
 
-template <int NDG>
+template <int NDG, bool kC>
 __global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaT<double> DA, DiaT<double> DT, IrArgs a) {
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
   double *sx = reinterpret_cast<double *>(ir_smem_raw);
@@ -1113,11 +1128,11 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaT<double> DA, 
     bool done = false;
     if constexpr (NDG == 5 || NDG == 7) {
       if (a.stencil && full) {
-        ir_quad_mv_st<double, double, NDG>(D, G, sv, r0, nr, li0, own, y);
+        ir_quad_mv_st<double, double, NDG, kC>(D, G, sv, r0, nr, li0, own, y);
         done = true;
       }
     }
-    if (!done) ir_quad_mv<double, double, NDG>(D, G, sv, r0, nr, li0, NDG > 0 ? NDG : D.nd, y);
+    if (!done) ir_quad_mv<double, double, NDG, kC>(D, G, sv, r0, nr, li0, NDG > 0 ? NDG : D.nd, y);
   };
 
   // start (x0 = 0): r = r* = p = p* = b, x = 0; (r, r) -> |b| and the
@@ -1274,10 +1289,10 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaT<double> DA, 
   }
 }
 
-template <int NDG>
+template <int NDG, bool kC>
 inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, const IrArgs &a, size_t smem,
                                int G, bool probe, bool *fits) {
-  auto fn = k_bicg_onchip<NDG>;
+  auto fn = k_bicg_onchip<NDG, kC>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (probe) {
@@ -1318,7 +1333,7 @@ inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, co
 //   C: p = beta p + r, q = beta q + s, (q, q) -> alpha = rs / (q, q).
 // Three grid reductions and no publication wait per iteration; element
 // operations are the engine's, only the dot sums' order differs.
-template <int NDG>
+template <int NDG, bool kC>
 __global__ void __launch_bounds__(kIrThreads, 1) k_cr_onchip(DiaT<double> D, IrArgs a) {
   using TW = IrWords<double>;
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
@@ -1393,11 +1408,11 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_cr_onchip(DiaT<double> D, IrA
     bool done = false;
     if constexpr (NDG == 5 || NDG == 7) {
       if (a.stencil && li0 + kIrQ <= nr) {
-        ir_quad_mv_st<double, double, NDG>(D, R, sr, r0, nr, li0, own4, y);
+        ir_quad_mv_st<double, double, NDG, kC>(D, R, sr, r0, nr, li0, own4, y);
         done = true;
       }
     }
-    if (!done) ir_quad_mv<double, double, NDG>(D, R, sr, r0, nr, li0, NDG > 0 ? NDG : D.nd, y);
+    if (!done) ir_quad_mv<double, double, NDG, kC>(D, R, sr, r0, nr, li0, NDG > 0 ? NDG : D.nd, y);
   };
   unsigned long long gen = 0;
   int code = kRunning;
@@ -1663,10 +1678,10 @@ inline bool ir_shape(const ks_ctx *ctx, long long n, IrShape *s, bool fill = fal
 
 // Cooperative launch of one CTA per SM; `probe`: only check that the grid
 // can be co-resident (sets *fits). `cls`: its class in a profiled solve.
-template <class VT, class MT, int NDG>
+template <class VT, class MT, int NDG, bool kC>
 inline cudaError_t ir_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
                                bool *fits, int cls) {
-  auto fn = k_cg_onchip<VT, MT, NDG>;
+  auto fn = k_cg_onchip<VT, MT, NDG, kC>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
   if (e != cudaSuccess) return e;
   if (probe) {
@@ -1691,18 +1706,26 @@ inline cudaError_t ir_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, co
   return cudaLaunchKernelEx(&cfg, fn, dview<MT>(A), a);
 }
 
+template <class VT, class MT, int NDG>
+inline cudaError_t ir_launch_c(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
+                               bool *fits, int cls) {
+  if constexpr (std::is_same<MT, double>::value)
+    if (A.dia_cst) return ir_launch_n<VT, MT, NDG, true>(ctx, A, a, sh, probe, fits, cls);
+  return ir_launch_n<VT, MT, NDG, false>(ctx, A, a, sh, probe, fits, cls);
+}
+
 template <class VT, class MT>
 inline cudaError_t ir_launch(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
                              bool *fits, int cls) {
-  if (A.dia_nd == 7) return ir_launch_n<VT, MT, 7>(ctx, A, a, sh, probe, fits, cls);
-  if (A.dia_nd == 5) return ir_launch_n<VT, MT, 5>(ctx, A, a, sh, probe, fits, cls);
-  return ir_launch_n<VT, MT, 0>(ctx, A, a, sh, probe, fits, cls);
+  if (A.dia_nd == 7) return ir_launch_c<VT, MT, 7>(ctx, A, a, sh, probe, fits, cls);
+  if (A.dia_nd == 5) return ir_launch_c<VT, MT, 5>(ctx, A, a, sh, probe, fits, cls);
+  return ir_launch_c<VT, MT, 0>(ctx, A, a, sh, probe, fits, cls);
 }
 
-template <int NDG>
+template <int NDG, bool kC>
 inline cudaError_t icr_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
                                 bool *fits) {
-  auto fn = k_cr_onchip<NDG>;
+  auto fn = k_cr_onchip<NDG, kC>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
   if (e != cudaSuccess) return e;
   if (probe) {

@@ -354,6 +354,8 @@ inline DiaT<MT> dview(const CsrDev &A) {
   d.cmax = A.dia_cmax;
   for (int k = 0; k < kMaxDiag; k++) d.off[k] = A.dia_off[k];
   d.quad = 0;
+  d.cst = std::is_same<MT, double>::value ? A.dia_cst : 0;
+  for (int k = 0; k < kMaxDiag; k++) d.cv[k] = (MT)(d.cst ? A.dia_cv[k] : 0.0);
   return d;
 }
 
@@ -402,6 +404,13 @@ inline void launch_spmv_dn(ks_ctx *ctx, const CsrDev &A, const GX &g0, const GX 
   if constexpr (NV == 1 && Epi::ND == 0 && (NDG == 5 || NDG == 7) && GX::kPlain && has_row4<Epi>::value &&
                 !std::is_same<MT, double>::value)
     dv.quad = dia_quad_ok(A, g0.x, epi.y) ? 1 : 0;
+  if constexpr (std::is_same<MT, double>::value) {
+    if (A.dia_cst) {  // on the same grid: sums in its epilogue add their terms in the same order
+      launch_k(ctx, spmv_dia_kernel<NV, NDG, MT, GX, Epi, true>, dim3(grid), dim3(kThreads), 0, dv, g0, g1, epi, stop,
+               red_of(ctx, slot));
+      return;
+    }
+  }
   launch_k(ctx, spmv_dia_kernel<NV, NDG, MT, GX, Epi>, dim3(grid), dim3(kThreads), 0, dv, g0, g1, epi, stop,
            red_of(ctx, slot));
 }

@@ -1010,9 +1010,13 @@ inline bool run_cr_onchip(const Env<double> &E, const double *b, double *x, doub
   bool fits = false;
   const IrArgs probe{};
   auto launch = [&](const IrArgs &a, bool pr) {
-    return A.dia_nd == 7 ? icr_launch_n<7>(ctx, A, a, sh, pr, &fits)
-                         : A.dia_nd == 5 ? icr_launch_n<5>(ctx, A, a, sh, pr, &fits)
-                                         : icr_launch_n<0>(ctx, A, a, sh, pr, &fits);
+    if (A.dia_cst)
+      return A.dia_nd == 7   ? icr_launch_n<7, true>(ctx, A, a, sh, pr, &fits)
+             : A.dia_nd == 5 ? icr_launch_n<5, true>(ctx, A, a, sh, pr, &fits)
+                             : icr_launch_n<0, true>(ctx, A, a, sh, pr, &fits);
+    return A.dia_nd == 7   ? icr_launch_n<7, false>(ctx, A, a, sh, pr, &fits)
+           : A.dia_nd == 5 ? icr_launch_n<5, false>(ctx, A, a, sh, pr, &fits)
+                           : icr_launch_n<0, false>(ctx, A, a, sh, pr, &fits);
   };
   if (launch(probe, true) != cudaSuccess || !fits) {
     (void)cudaGetLastError();
@@ -1184,9 +1188,15 @@ inline void launch_pair_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, const d
   const long long need = ((long long)A.n + kThreads - 1) / kThreads;
   const long long wave = (long long)ctx->num_sms * spmv_dia_ctas_per_sm<1, NDG, double, GPtr<double>, EpiA>(ctx->device);
   ctx->next_class = kMv;
-  launch_k(ctx, spmv_dia_pair_kernel<NDG, GPtr<double>, Epi>,
-           dim3((unsigned)std::max<long long>(1, std::min(need, wave))), dim3(kThreads), 0, dview<double>(A),
-           dview_mirror(A, T), GPtr<double>{p}, GPtr<double>{ps}, epi, stop, red_of(ctx, 0));
+  const dim3 grid((unsigned)std::max<long long>(1, std::min(need, wave)));
+  auto run = [&](auto kern) {
+    launch_k(ctx, kern, grid, dim3(kThreads), 0, dview<double>(A), dview_mirror(A, T), GPtr<double>{p}, GPtr<double>{ps},
+             epi, stop, red_of(ctx, 0));
+  };
+  if (A.dia_cst && T.dia_cst)
+    run(spmv_dia_pair_kernel<NDG, GPtr<double>, Epi, true>);
+  else
+    run(spmv_dia_pair_kernel<NDG, GPtr<double>, Epi, false>);
 }
 
 template <class EpiA, class Epi>
@@ -1319,9 +1329,13 @@ inline bool run_bicg_onchip(const Env<double> &E, const double *b, double *x, do
   if (2 * E.ld < E.n + 2 * pad) return false;
   bool fits = false;
   auto launch = [&](const IrArgs &a, bool pr) {
-    return A.dia_nd == 7 ? ib_launch_n<7>(ctx, A, T, a, smem, (int)G, pr, &fits)
-                         : A.dia_nd == 5 ? ib_launch_n<5>(ctx, A, T, a, smem, (int)G, pr, &fits)
-                                         : ib_launch_n<0>(ctx, A, T, a, smem, (int)G, pr, &fits);
+    if (A.dia_cst && T.dia_cst)
+      return A.dia_nd == 7   ? ib_launch_n<7, true>(ctx, A, T, a, smem, (int)G, pr, &fits)
+             : A.dia_nd == 5 ? ib_launch_n<5, true>(ctx, A, T, a, smem, (int)G, pr, &fits)
+                             : ib_launch_n<0, true>(ctx, A, T, a, smem, (int)G, pr, &fits);
+    return A.dia_nd == 7   ? ib_launch_n<7, false>(ctx, A, T, a, smem, (int)G, pr, &fits)
+           : A.dia_nd == 5 ? ib_launch_n<5, false>(ctx, A, T, a, smem, (int)G, pr, &fits)
+                           : ib_launch_n<0, false>(ctx, A, T, a, smem, (int)G, pr, &fits);
   };
   const IrArgs probe{};
   if (launch(probe, true) != cudaSuccess || !fits) {
