@@ -1,12 +1,14 @@
 // Instantiations and launches of the CG with the matrix on chip
-// (ks_chip_cg.cuh).
-#include "ks_chip_cg.cuh"
+// (ks_chip_cg.cuh) and on tiles (ks_tile_cg.cuh).
+#include "ks_tile_cg.cuh"
 
 namespace ks {
 
-template <class VT, int NDG, int RJ, bool kTile>
-static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
-  auto fn = k_cg_chip<VT, NDG, RJ, kTile>;
+// A cooperative launch of fn(args...), or with `probe` only the check that it
+// can be co-resident.
+template <class... KArgs, class... Args>
+static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShape &sh, bool probe, bool *fits, int cls,
+                               const Args &...args) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
   if (e != cudaSuccess) return e;
   if (probe) {
@@ -27,7 +29,12 @@ static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape
   cfg.numAttrs = 1;
   ctx->launches++;
   ProfLaunch pl(ctx, cls);
-  return cudaLaunchKernelEx(&cfg, fn, a);
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+template <class VT, int NDG, int RJ, bool kTile>
+static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
+  return coop_launch(ctx, k_cg_chip<VT, NDG, RJ, kTile>, sh, probe, fits, cls, a);
 }
 
 template <class VT, int NDG, bool kTile>
@@ -52,6 +59,13 @@ cudaError_t chip_launch_f64(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh,
 }
 cudaError_t chip_launch_f32(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
   return chip_launch_t<float>(ctx, a, sh, probe, fits, cls);
+}
+
+cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits,
+                        int cls) {
+  TileDiag D{};
+  for (int k = 0; k < 7; k++) D.v[k] = A.dia_cv[k];
+  return coop_launch(ctx, k_cg_tile, sh, probe, fits, cls, a, D);
 }
 
 }  // namespace ks

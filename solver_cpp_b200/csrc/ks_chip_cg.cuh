@@ -867,4 +867,54 @@ inline cudaError_t chip_launch(ks_ctx *ctx, const ChipArgs &a, const ChipShape &
   return sizeof(VT) == 8 ? chip_launch_f64(ctx, a, sh, probe, fits, cls) : chip_launch_f32(ctx, a, sh, probe, fits, cls);
 }
 
+// ---------------------------------------------------------------- CG on tiles
+// Shape and launch of k_cg_tile (ks_tile_cg.cuh).
+constexpr int kTileRows = 32;  // rows per thread: 64 words of TMEM each for r and x
+constexpr int kTileHaloThreads = kChipThreads - 32;  // warps 1 .. 15
+constexpr int kTileHaloZ = 3, kTileHaloY = 4;  // columns of a z face, rows of a y face per thread of them at most
+
+// The tile with the least work (the rows its threads walk, plus half a row for
+// each of the halo's) on at most one CTA per SM; false where none fits on chip.
+inline bool tile_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShape *s) {
+  const long long sms = std::min(ctx->num_sms, (int)kChipMaxGrid);
+  if (A.dia_box < 2 || !A.dia_cst || A.dia_cmin != 0 || A.dia_cmax != n || n > sms * kTileRows * kChipThreads) return false;
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  *s = ChipShape{};
+  s->tile = 1;
+  s->nx = A.dia_off[5];
+  s->ny = A.dia_off[6] / s->nx;
+  s->nz = (int)(n / A.dia_off[6]);
+  double best = 0.0;
+  for (int by = 1; by <= s->ny; by++) {
+    const long long gy = (s->ny + by - 1) / by;
+    if (gy > sms) continue;
+    const long long bz = (s->nz + sms / gy - 1) / (sms / gy);
+    const long long elems = 2 + (long long)(s->nx + 1) * (by + 2) * (bz + 2);
+    const long long halo = 2LL * s->nx * (by + bz), cols = ((long long)s->nx * by + kChipThreads - 1) / kChipThreads;
+    const double cost = (double)(cols * ((bz + 7) / 8 * 8)) * kChipThreads + 0.5 * (double)halo;
+    if (cols * ((bz + 7) / 8 * 8) > kTileRows || (long long)s->nx * by > kTileHaloZ * kTileHaloThreads ||
+        s->nx * bz > kTileHaloY * kTileHaloThreads || elems > (1 << 20) ||
+        sizeof(double) * (size_t)elems + 2048 > (size_t)optin || (best > 0.0 && cost >= best))
+      continue;
+    best = cost;
+    s->by = by;
+    s->bz = (int)bz;
+    s->gy = (int)gy;
+    s->elems = (int)elems;
+    s->smem = sizeof(double) * (size_t)elems;
+  }
+  if (best == 0.0) return false;
+  s->G = s->gy * ((s->nz + s->bz - 1) / s->bz);
+  return true;
+}
+
+// One launch (`probe`: only check that the grid can be co-resident, *fits);
+// `cls`: its class in a profiled solve. ks_chip_cg.cu.
+cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits,
+                        int cls);
+
 }  // namespace ks

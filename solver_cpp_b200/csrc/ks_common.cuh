@@ -104,7 +104,8 @@ struct CsrDev {
   // of n elements (dia_ds = n, dia_pad = 0).
   int dia_sym = 0;
   // 1: a 7-point stencil on a box of lines of dia_off[5] rows and planes of
-  // dia_off[6] rows, without an entry across the end of a line or plane.
+  // dia_off[6] rows, without an entry across the end of a line or plane; 2: and
+  // with every entry inside the box.
   int dia_box = 0;
   int dia_pad = 0;
   long long dia_ds = 0;

@@ -353,12 +353,13 @@ static void free_dia(CsrDev &A) {
   A.dia_ds = 0;
 }
 
-// Sets *bad if a row at the end of a line (b rows) or of a plane (c rows) has
-// an entry on the diagonal that leaves it: mask bits 0..6 are the diagonals
-// -c, -b, -1, 0, 1, b, c.
+// Sets f->bad if a row at the end of a line (b rows) or of a plane (c rows)
+// has an entry on the diagonal that leaves it (mask bits 0..6 are the diagonals
+// -c, -b, -1, 0, 1, b, c), f->gap if a row lacks an entry inside the box.
 struct DiagFacts {
   unsigned long long lo[kMaxDiag], hi[kMaxDiag];  // least and greatest bit pattern of each diagonal's entries
   int bad;  // entries across the end of a line or plane
+  int gap;  // entries inside the box that are absent
 };
 __global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, int b, int c, DiagFacts *f) {
   const int ny = c / b;
@@ -370,6 +371,9 @@ __global__ void k_dia_boxcheck(const unsigned char *__restrict__ mask, int n, in
     if (y == 0) out |= 1u << 1;
     if (y == ny - 1) out |= 1u << 5;
     if (mask[i] & out) f->bad = 1;
+    if (i < c) out |= 1u;
+    if (i >= n - c) out |= 1u << 6;
+    if ((mask[i] | out) != 0x7fu) f->gap = 1;
   }
 }
 
@@ -541,7 +545,7 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   A.dia_cmin = (int)cmin;
   A.dia_cmax = (int)cmax;
   A.dia_sym = sym ? 1 : 0;
-  A.dia_box = box ? 1 : 0;
+  A.dia_box = box ? (f.gap ? 1 : 2) : 0;
   A.dia_cst = cst ? 1 : 0;
   for (int k = 0; k < kMaxDiag; k++) {
     A.dia_cv[k] = 0.0;
@@ -787,7 +791,7 @@ ks_status ks_ctx_create(int device, ks_ctx **out) {
   std::memset(ctx->h_snap, 0, sizeof(int) * ctx->nflags);
   if (cudaMalloc(&ctx->d_stage, sizeof(double) * kStageLen) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
   // barrier state of the on-chip kernels (ir_sync_bytes of one CTA per SM)
-  if (cudaMalloc(&ctx->ir_sync, 64 + 40 * (size_t)ctx->num_sms) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
+  if (cudaMalloc(&ctx->ir_sync, 64 + 72 * (size_t)ctx->num_sms) != cudaSuccess) return fail(KS_OUT_OF_MEMORY);
   ctx->flag_events = new cudaEvent_t[ctx->nflags];
   for (int i = 0; i < ctx->nflags; i++) {
     if (cudaEventCreateWithFlags(&ctx->flag_events[i], cudaEventDisableTiming) != cudaSuccess)

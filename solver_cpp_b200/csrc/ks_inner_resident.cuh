@@ -56,7 +56,8 @@ constexpr int kIrMaxSums = 2;    // values one reduction carries
 
 // Barrier state in device memory, zeroed before every launch: the grid
 // reductions' arrival counter, one publication flag per CTA, then the tagged
-// slots of k_cg_chip's reductions (two per CTA, ks_chip_cg.cuh).
+// slots of k_cg_chip's reductions (two per CTA, ks_chip_cg.cuh) and k_cg_tile's
+// flags (32 bytes apart, ks_tile_cg.cuh).
 struct IrSync {
   unsigned long long count;  // CTA arrivals at the reductions, all generations
   unsigned long long reserved;
@@ -70,7 +71,7 @@ __device__ __forceinline__ unsigned long long *ir_pub(IrSync *s, int q) {
 
 inline size_t ir_sync_bytes(int G) {
   return sizeof(IrSync) + sizeof(unsigned long long) * (size_t)((G + 1) & ~1) +
-         sizeof(ulonglong2) * 2 * (size_t)G;
+         (2 * sizeof(ulonglong2) + 32) * (size_t)G;
 }
 
 struct IrArgs {

@@ -807,27 +807,38 @@ constexpr long long kChipMinRows = 8192;
 
 // Larger systems whose matrix fits on chip across the GPU as well as their
 // vectors (up to about 4,096 rows per SM in FP64, one GPU, a diagonal copy;
-// ks_params.cluster_solve 0): the whole solve as one cooperative kernel
-// (k_cg_chip, ks_chip_cg.cuh). Returns false, having launched nothing, when
-// the system does not qualify.
+// ks_params.cluster_solve 0), or constant-coefficient 7-point stencils on a box
+// whose vectors do (up to about 16,000 rows per SM): the whole solve as one cooperative kernel
+// (k_cg_chip, ks_chip_cg.cuh; k_cg_tile, ks_tile_cg.cuh). Returns false, having
+// launched nothing, when the system does not qualify.
 inline bool run_cg_chip(const Env<double> &E, const double *b, double *x, double *R, ks_status *s) {
   if (E.sp.cluster_solve || !E.outer || E.comm || E.mvals != KS_FP64 || !E.A->dia_nd || !E.A->dia_val) return false;
+  if (reinterpret_cast<uintptr_t>(R) % 16) return false;  // R takes the first two workspace slots
   ks_ctx *ctx = E.ctx;
   ChipShape sh;
-  // R takes the first two workspace slots
-  if (!chip_shape<double>(ctx, *E.A, E.n, &sh) || reinterpret_cast<uintptr_t>(R) % 16) return false;
-  const IrArgs ir{b, x, R, E.st, nullptr, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns, (int)E.n, sh.rpc, sh.rj, 1, 0};
-  const ChipArgs a = chip_args<double, double>(*E.A, ir, sh, 0);
-  bool fits = false;
-  if (chip_launch<double>(ctx, a, sh, true, &fits, 0) != cudaSuccess || !fits) {
+  const IrArgs ir{b, x, R, E.st, nullptr, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns, (int)E.n, 0, 0,
+                  1, 0};
+  ChipArgs a;
+  // the matrix on chip (k_cg_chip), else the vectors alone on tiles (k_cg_tile)
+  bool tiles = false;
+  auto launch = [&](bool probe, bool *fits, int cls) {
+    return tiles ? tile_launch(ctx, *E.A, a, sh, probe, fits, cls) : chip_launch<double>(ctx, a, sh, probe, fits, cls);
+  };
+  for (int way = 0;; way++) {
+    if (way == 2) return false;
+    tiles = way == 1;
+    if (!(tiles ? tile_shape(ctx, *E.A, E.n, &sh) : chip_shape<double>(ctx, *E.A, E.n, &sh))) continue;
+    a = chip_args<double, double>(*E.A, ir, sh, 0);
+    bool fits = false;
+    if (launch(true, &fits, 0) == cudaSuccess && fits) break;
     (void)cudaGetLastError();
-    return false;
   }
   launch_scalar(ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
   cudaError_t e = cudaMemsetAsync(ctx->ir_sync, 0, ir_sync_bytes(sh.G), ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(R, 0, chip_r_bytes<double>(E.n), ctx->stream);
+  if (e == cudaSuccess && !tiles) e = cudaMemsetAsync(R, 0, chip_r_bytes<double>(E.n), ctx->stream);
   // a profiled solve counts the whole solve as one SpMV-class launch
-  if (e == cudaSuccess) e = chip_launch<double>(ctx, a, sh, false, &fits, kMv);
+  bool fits = false;
+  if (e == cudaSuccess) e = launch(false, &fits, kMv);
   *s = e == cudaSuccess ? KS_OK : cuda_fail(ctx, e, "on-chip CG launch");
   return true;
 }
@@ -2379,7 +2390,7 @@ struct InnerRunner {
   IrShape sh{};
   bool chip = false;  // the matrix on chip too (k_cg_chip)
   ChipShape csh{};
-  unsigned long long tag = 0;  // the last tag used on fb.P
+  unsigned long long tag = 0;  // the last tag used on fb.P (k_cg_chip)
   ChipArgs chip_args(const IrArgs &a) const {
     return iprec == KS_BF16 ? ks::chip_args<float, __nv_bfloat16>(*E32.A, a, csh, tag)
                             : ks::chip_args<float, float>(*E32.A, a, csh, tag);
@@ -2423,8 +2434,10 @@ void InnerRunner<VT>::setup_resident() {
   if (iprec == KS_FP32 ? !E32.A->dia_val32 : !E32.A->dia_val16) return;
   if (vec_count(KS_CG, E32.sp, E32.n, sizeof(float), ctx->l2_bytes) < 3) return;  // P (two slots) and r
   bool fits = false;
+  // the published r with its tags takes the first two slots
   if (E32.sp.maxloop < (1ll << 31) && chip_shape<float>(ctx, *E32.A, E32.n, &csh) &&
-      reinterpret_cast<uintptr_t>(Ws<float>{ws32, E32.ld, E32.off}.take()) % 8 == 0 && chip_launch<float>(ctx, chip_args(IrArgs{}), csh, true, &fits, 0) == cudaSuccess && fits) {
+      reinterpret_cast<uintptr_t>(Ws<float>{ws32, E32.ld, E32.off}.take()) % 8 == 0 &&
+      chip_launch<float>(ctx, chip_args(IrArgs{}), csh, true, &fits, 0) == cudaSuccess && fits) {
     Ws<float> W{ws32, E32.ld, E32.off};
     fb.P = W.take(2);
     fb.r = W.take();

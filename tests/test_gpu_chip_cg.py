@@ -142,3 +142,46 @@ def test_inner_cg_of_another_length(ks, ctx):
         step = ks.solve(ctx, M, "VPCG", b, inner_fast=1, **kw)
         assert chip.status == step.status == 0 and np.array_equal(chip.x, step.x)
     M.close()
+
+
+# boxes whose matrix does not fit on chip (k_cg_tile): tiles that divide the
+# box and ones that do not, long and short lines, the largest that fit
+TILES64 = [(91, 90, 89), (128, 128, 128), (130, 127, 129), (300, 60, 61), (9, 300, 301), (1200, 40, 33)]
+
+
+@pytest.mark.parametrize("shape", TILES64)
+@pytest.mark.parametrize("const", [False, True])
+def test_fp64_tiles_against_engine(ks, ctx, shape, const):
+    if const:
+        from solver_cpp_b200.matrices import poisson3d
+
+        A = poisson3d(*shape)
+        A.val[A.val > 0] = 6.3  # 5 % dominant, as the random ones
+    else:
+        A = box(*shape)
+    chip, step = both(ks, ctx, A, L=30)
+    assert chip.report["n_mv"] == 1 and chip.report["n_dot"] == 0, chip.report
+    agree(chip, step)
+
+
+def test_fp64_tiles_unsymmetric_and_with_gaps(ks, ctx):
+    """The full layout; and constant values with entries missing inside the box."""
+    chip, step = both(ks, ctx, box(93, 91, 90, skew=0.02), L=15)
+    agree(chip, step)
+    nx, ny, nz = 93, 91, 90
+
+    def some(i, o):
+        inside = (i % nx < nx - 1) if o == 1 else (((i // nx) % ny < ny - 1) if o == nx else np.ones(len(i), bool))
+        return inside & (i % 7 != 3)
+
+    A = banded(nx * ny * nz, [-nx * ny, -nx, -1, 0, 1, nx, nx * ny], keep=some)
+    off = A.val < 0
+    A.val[off], A.val[~off] = -1.0, 6.3
+    chip, step = both(ks, ctx, A, L=30)
+    agree(chip, step)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "bf16"])
+@pytest.mark.parametrize("shape", [(109, 108, 107), (131, 128, 127), (160, 160, 160), (700, 45, 44)])
+def test_inner_tiles_bitwise(ks, ctx, shape, prec):
+    test_inner_cg_bitwise(ks, ctx, shape, prec)
