@@ -1,5 +1,6 @@
 // Instantiations and launches of the CG with the matrix on chip
-// (ks_chip_cg.cuh) and on tiles (ks_tile_cg.cuh).
+// (ks_chip_cg.cuh), on tiles (ks_tile_cg.cuh) and of CSR matrices (ks_csr_cg.cuh).
+#include "ks_csr_cg.cuh"
 #include "ks_tile_cg.cuh"
 
 namespace ks {
@@ -8,18 +9,18 @@ namespace ks {
 // can be co-resident.
 template <class... KArgs, class... Args>
 static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShape &sh, bool probe, bool *fits, int cls,
-                               const Args &...args) {
+                               int threads, const Args &...args) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
   if (e != cudaSuccess) return e;
   if (probe) {
     int b = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kChipThreads, sh.smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, sh.smem);
     *fits = e == cudaSuccess && b >= 1;
     return e;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(sh.G);
-  cfg.blockDim = dim3(kChipThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = sh.smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute at[1];
@@ -34,7 +35,7 @@ static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShap
 
 template <class VT, int NDG, int RJ, bool kTile>
 static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
-  return coop_launch(ctx, k_cg_chip<VT, NDG, RJ, kTile>, sh, probe, fits, cls, a);
+  return coop_launch(ctx, k_cg_chip<VT, NDG, RJ, kTile>, sh, probe, fits, cls, kChipThreads, a);
 }
 
 template <class VT, int NDG, bool kTile>
@@ -65,7 +66,13 @@ cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const C
                         int cls) {
   TileDiag D{};
   for (int k = 0; k < 7; k++) D.v[k] = A.dia_cv[k];
-  return coop_launch(ctx, k_cg_tile, sh, probe, fits, cls, a, D);
+  return coop_launch(ctx, k_cg_tile, sh, probe, fits, cls, kChipThreads, a, D);
+}
+
+cudaError_t csr_launch(ks_ctx *ctx, const CsrCgArgs &a, const CsrShape &sh, bool probe, bool *fits, int cls) {
+  auto run = [&](auto kern) { return coop_launch(ctx, kern, sh, probe, fits, cls, sh.threads, a); };
+  if (sh.threads == 1024) return run(k_cg_csr<1024, 4>);  // more than 2,048 rows per CTA
+  return sh.rj == 1 ? run(k_cg_csr<512, 1>) : sh.rj == 2 ? run(k_cg_csr<512, 2>) : run(k_cg_csr<512, 4>);
 }
 
 }  // namespace ks

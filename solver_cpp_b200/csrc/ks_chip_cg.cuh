@@ -67,6 +67,12 @@ __device__ __forceinline__ ulonglong2 *ir_slots(IrSync *s, unsigned G, unsigned 
   return base + (size_t)(gen & 1) * G;
 }
 
+// The publication flag of CTA q, 32 bytes apart, behind the reductions' slots.
+__device__ __forceinline__ unsigned long long *tile_flag(IrSync *s, int q) {
+  return reinterpret_cast<unsigned long long *>(ir_slots(s, gridDim.x, 0) + 2 * gridDim.x) + 4 * q;
+}
+
+
 // A value and its tag as one 16-byte access (single-copy atomic).
 __device__ __forceinline__ void chip_slot_st(ulonglong2 *q, double v, unsigned long long tag) {
   const unsigned long long lo = (unsigned long long)__double_as_longlong(v);
@@ -127,8 +133,9 @@ struct ChipClock {
 // CTA has posted g + 1, i.e. after every CTA has read generation g's.
 constexpr unsigned kChipDirect = 32;
 
+template <int kThreadsPerCta = kChipThreads>
 __device__ __forceinline__ void chip_post(const IrArgs &a, unsigned long long gen, double v) {
-  constexpr int kWarps = kChipThreads / 32;
+  constexpr int kWarps = kThreadsPerCta / 32;
   __shared__ double sh[kWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   v = warp_sum(v);
@@ -916,5 +923,46 @@ inline bool tile_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShap
 // `cls`: its class in a profiled solve. ks_chip_cg.cu.
 cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits,
                         int cls);
+
+// ---------------------------------------------------------------- CG, CSR
+// Shape and launch of k_cg_csr (ks_csr_cg.cuh).
+constexpr int kCsrRows = 4;  // rows per thread at most (of 512 threads, above 2,048 rows per CTA of 1,024)
+
+struct CsrCgArgs : IrArgs {  // P is the array R of published r
+  const int *ptr, *slice;
+  const double *val;
+  const short *off;
+  int wl, wu;
+};
+
+struct CsrShape : ChipShape {
+  int threads = 0;
+  int wl = 0, wu = 0;
+};
+
+// The CTAs of chip_ctas. False
+// where the matrix has no slices or its window does not fit.
+inline bool csr_shape(const ks_ctx *ctx, const CsrDev &A, long long n, CsrShape *s) {
+  const long long sms = std::min(ctx->num_sms, (int)kChipMaxGrid);
+  if (!A.sell_val || n < 1 || n != A.n || n > sms * kCsrRows * 1024) return false;
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  *s = CsrShape{};
+  const long long G = chip_ctas(n, sms);
+  s->rpc = (int)(((n + G - 1) / G + 31) / 32 * 32);
+  s->G = (int)((n + s->rpc - 1) / s->rpc);
+  s->rj = 1;
+  s->threads = s->rpc <= kCsrRows * 512 ? 512 : 1024;
+  while (s->rj * s->threads < s->rpc) s->rj *= 2;
+  s->wl = A.sell_lo;
+  s->wu = A.sell_hi;
+  s->smem = sizeof(double) * ((size_t)s->rpc + s->wl + s->wu);
+  return s->rj <= kCsrRows && s->smem + 2048 <= (size_t)optin;
+}
+
+cudaError_t csr_launch(ks_ctx *ctx, const CsrCgArgs &a, const CsrShape &sh, bool probe, bool *fits, int cls);
 
 }  // namespace ks

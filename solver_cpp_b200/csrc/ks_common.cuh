@@ -21,6 +21,7 @@ constexpr int kPad = 8;             // tail padding of col/val arrays (elements)
 constexpr int kMaxDots = 8;         // simultaneous reductions in one kernel
 constexpr int kBlockDotGroup = 8;   // tall-skinny dots per pass
 constexpr int kMaxGroups = 128;     // block-dot groups in one launch (1024 dots)
+constexpr int kSliceMinRows = 8192;  // matrices of more rows get slices (CsrDev::sell_*)
 constexpr int kMaxDiag = 8;         // diagonals of a matrix's diagonal copy (8-bit row masks)
 
 // ---------------------------------------------------------------- state
@@ -79,6 +80,16 @@ struct CsrDev {
   int *rb = nullptr;  // row-block boundaries, nrb + 1 entries
   int4 *rbi = nullptr;  // per row block: first row, end row, first nonzero, end nonzero
   int nrb = 0;
+  // Copy of the FP64 matrix in slices of 32 rows for k_cg_csr (ks_csr_cg.cuh):
+  // entry k of row 32 s + l is element 32 (sell_ptr[s] + k) + l of sell_val and
+  // sell_off (col - row). Kept for matrices without a diagonal copy, up to 4,096
+  // rows per SM, whose offsets fit in 16 bits and whose slices hold no more than
+  // twice the nonzeros; sell_lo, sell_hi: the largest offsets below and above
+  // the row. Null otherwise.
+  int *sell_ptr = nullptr;
+  double *sell_val = nullptr;
+  short *sell_off = nullptr;
+  int sell_lo = 0, sell_hi = 0;
   // Diagonal copy of a stencil-like matrix, read by the SpMV instead of the
   // CSR arrays: every row holds its columns at offsets (col - row) from a set
   // of dia_nd <= kMaxDiag offsets, dia_off ascending. Values are stored

@@ -556,6 +556,83 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   return KS_OK;
 }
 
+// The slices of k_cg_csr (CsrDev::sell_*): one warp per slice of 32 rows, lane =
+// row. range: the largest offset below and above a row.
+__global__ void k_sell_fill(const int *__restrict__ ptr, const short *__restrict__ col16, const double *__restrict__ val,
+                            int n, const int *__restrict__ slice, double *__restrict__ sval, short *__restrict__ soff,
+                            int *range) {
+  int lo = 0, hi = 0;
+  const int lane = threadIdx.x & 31, warps = gridDim.x * blockDim.x / 32;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < (n + 31) / 32; s += warps) {
+    const int i = 32 * s + lane, j0 = i < n ? ptr[i] : 0, len = i < n ? ptr[i + 1] - j0 : 0;
+    const int m = slice[s + 1] - slice[s];
+    for (int k = 0; k < m; k++) {
+      const long long e = 32LL * (slice[s] + k) + lane;
+      const int o = k < len ? col16[j0 + k] : 0;
+      sval[e] = k < len ? val[j0 + k] : 0.0;
+      soff[e] = (short)o;
+      lo = max(lo, -o);
+      hi = max(hi, o);
+    }
+  }
+  for (int d = 16; d > 0; d >>= 1) {
+    lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+  }
+  if (lane == 0) {
+    atomicMax(range, lo);
+    atomicMax(range + 1, hi);
+  }
+}
+
+// An optimisation: where the device cannot hold the copy there is none.
+static ks_status build_slices(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr) {
+  const int ns = (A.n + 31) / 32;
+  std::vector<int> sp((size_t)ns + 1, 0);
+  for (int s = 0; s < ns; s++) {
+    int m = 0;
+    for (int i = 32 * s; i < std::min(A.n, 32 * s + 32); i++) m = std::max(m, host_ptr[i + 1] - host_ptr[i]);
+    const long long next = (long long)sp[s] + m;
+    if (32 * next > std::min(2 * A.nnz + 1024, (1LL << 31) - 1)) return KS_OK;
+    sp[s + 1] = (int)next;
+  }
+  const size_t total = 32 * (size_t)sp[ns];
+  int *range = nullptr;
+  int h[2] = {0, 0};
+  cudaError_t e = cudaMalloc(&A.sell_ptr, sizeof(int) * sp.size());
+  if (e == cudaSuccess) e = cudaMalloc(&A.sell_off, sizeof(short) * std::max<size_t>(total, 1));
+  if (e == cudaSuccess) e = cudaMalloc(&A.sell_val, sizeof(double) * std::max<size_t>(total, 1));
+  if (e == cudaSuccess) e = cudaMalloc(&range, sizeof(h));
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+  } else {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(A.sell_ptr, sp.data(), sizeof(int) * sp.size(), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(range, 0, sizeof(h), ctx->stream);
+    if (e == cudaSuccess) {
+      k_sell_fill<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(A.ptr, A.col16, A.val, A.n, A.sell_ptr, A.sell_val, A.sell_off,
+                                                            range);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, range, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // sp goes out of scope, too
+    if (e != cudaSuccess) {
+      cudaFree(range);
+      return cuda_fail(ctx, e, "matrix slices");
+    }
+    A.sell_lo = h[0];
+    A.sell_hi = h[1];
+    cudaFree(range);
+    return KS_OK;
+  }
+  cudaFree(A.sell_ptr);
+  cudaFree(A.sell_off);
+  cudaFree(A.sell_val);
+  A.sell_ptr = nullptr;
+  A.sell_off = nullptr;
+  A.sell_val = nullptr;
+  return KS_OK;
+}
+
 static void free_csr(CsrDev &A) {
   free_dia(A);
   cudaFree(A.ptr);
@@ -566,6 +643,9 @@ static void free_csr(CsrDev &A) {
   cudaFree(A.val16);
   cudaFree(A.rb);
   cudaFree(A.rbi);
+  cudaFree(A.sell_ptr);
+  cudaFree(A.sell_val);
+  cudaFree(A.sell_off);
   A = CsrDev();
 }
 
@@ -630,6 +710,8 @@ static ks_status finish_csr(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr, uns
   }
   KS_CUDA(ctx, cudaGetLastError());
   if (!(flags & KS_MAT_NO_DIAG)) KS_TRY(build_diagonals(ctx, A, flags, cmin, cmax));
+  if (!A.dia_nd && A.col16 && cmin == 0 && cmax == A.n && A.n > kSliceMinRows && A.n <= 4096LL * ctx->num_sms)
+    KS_TRY(build_slices(ctx, A, host_ptr));
   // rb and rbi are host vectors going out of scope: the copies must complete first.
   KS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return KS_OK;

@@ -843,6 +843,38 @@ inline bool run_cg_chip(const Env<double> &E, const double *b, double *x, double
   return true;
 }
 
+// Matrices without a diagonal copy whose rows' columns lie near the row: the
+// whole solve as one cooperative kernel (k_cg_csr, ks_csr_cg.cuh; one GPU, FP64,
+// ks_params.cluster_solve 0). Returns false, having launched nothing, when the
+// system does not qualify.
+inline bool run_cg_csr(const Env<double> &E, const double *b, double *x, double *R, ks_status *s) {
+  if (E.sp.cluster_solve || !E.outer || E.comm || E.mvals != KS_FP64) return false;
+  ks_ctx *ctx = E.ctx;
+  const CsrDev &A = *E.A;
+  CsrShape sh;
+  if (!csr_shape(ctx, A, E.n, &sh)) return false;
+  CsrCgArgs a{};
+  static_cast<IrArgs &>(a) = IrArgs{b, x, R, E.st, nullptr, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns,
+                                    (int)E.n, sh.rpc, sh.rj, 1, 0};
+  a.ptr = A.ptr;
+  a.slice = A.sell_ptr;
+  a.val = A.sell_val;
+  a.off = A.sell_off;
+  a.wl = sh.wl;
+  a.wu = sh.wu;
+  bool fits = false;
+  if (csr_launch(ctx, a, sh, true, &fits, 0) != cudaSuccess || !fits) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  launch_scalar(ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
+  cudaError_t e = cudaMemsetAsync(ctx->ir_sync, 0, ir_sync_bytes(sh.G), ctx->stream);
+  // a profiled solve counts the whole solve as one SpMV-class launch
+  if (e == cudaSuccess) e = csr_launch(ctx, a, sh, false, &fits, kMv);
+  *s = e == cudaSuccess ? KS_OK : cuda_fail(ctx, e, "on-chip CSR CG launch");
+  return true;
+}
+
 // Larger systems whose vectors fit on chip across the GPU (up to about 14,400
 // rows per SM in FP64, one GPU, a diagonal copy; ks_params.cluster_solve 0):
 // the whole solve as one cooperative kernel of one CTA per SM, r and q in
@@ -884,6 +916,7 @@ ks_status run_cg(const Env<VT> &E, const VT *b, VT *x, VT *ws, double *dws) {
   if constexpr (std::is_same<VT, double>::value) {
     ks_status s = KS_OK;
     if (E.n > kChipMinRows && run_cg_chip(E, b, x, ws, &s)) return s;
+    if (run_cg_csr(E, b, x, ws, &s)) return s;
     if (run_cg_resident(E, b, x, &s)) return s;
     if (run_cg_onchip(E, b, x, ws, &s)) return s;
   }

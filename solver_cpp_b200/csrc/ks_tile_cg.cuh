@@ -105,11 +105,6 @@ struct TileBlock {
   }
 };
 
-// The publication flag of CTA q, 32 bytes apart, behind the reductions' slots.
-__device__ __forceinline__ unsigned long long *tile_flag(IrSync *s, int q) {
-  return reinterpret_cast<unsigned long long *>(ir_slots(s, gridDim.x, 0) + 2 * gridDim.x) + 4 * q;
-}
-
 __device__ __forceinline__ void tile_halo_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kTileHaloThreads) : "memory"); }
 
 struct TileDiag {  // the diagonals' values
