@@ -419,8 +419,9 @@ __global__ void k_dia_range(const double *__restrict__ dval, const unsigned char
 static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long long cmin, long long cmax) {
   if (A.n < 1 || A.nnz < 1) return KS_OK;
   const int g = ctx->num_sms * 8;
-  int *d_buf = nullptr;  // kMaxDiag offsets, then the flags
-  KS_CUDA(ctx, cudaMalloc(&d_buf, sizeof(int) * (kMaxDiag + 1)));
+  int *d_buf = nullptr;  // kMaxDiag offsets and the flags; behind them the facts
+  constexpr size_t kFactsAt = 16 * ((sizeof(int) * (kMaxDiag + 1) + 15) / 16);
+  KS_CUDA(ctx, cudaMalloc(&d_buf, kFactsAt + sizeof(DiagFacts)));
   int h_buf[kMaxDiag + 1];
   for (int k = 0; k < kMaxDiag; k++) h_buf[k] = kDiagEmpty;
   h_buf[kMaxDiag] = 0;
@@ -488,10 +489,9 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
              o.off[6] > o.off[5] && o.off[6] % o.off[5] == 0 && A.n % o.off[6] == 0;
   for (int k = 0; box && k < 3; k++) box = o.off[k] == -o.off[6 - k];
   DiagFacts f{};
-  DiagFacts *d_f = nullptr;
-  e = cudaMalloc(&d_f, sizeof(f));
+  DiagFacts *const d_f = reinterpret_cast<DiagFacts *>(reinterpret_cast<char *>(d_buf) + kFactsAt);
   for (int k = 0; k < kMaxDiag; k++) f.lo[k] = ~0ull;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_f, &f, sizeof(f), cudaMemcpyHostToDevice, ctx->stream);
+  e = cudaMemcpyAsync(d_f, &f, sizeof(f), cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) {
     if (box) k_dia_boxcheck<<<g, 256, 0, ctx->stream>>>(A.dia_mask, A.n, o.off[5], o.off[6], d_f);
     k_dia_range<<<g, 256, 0, ctx->stream>>>(A.dia_val, A.dia_mask, A.n, o.nd, d_f);
@@ -499,7 +499,6 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(&f, d_f, sizeof(f), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d_f);
   if (e != cudaSuccess) {
     cudaFree(d_buf);
     return cuda_fail(ctx, e, "diagonal facts");

@@ -73,10 +73,13 @@ __global__ void __launch_bounds__(kThreads)
 // k basis vectors (GMRES's w -= sum h_i v_i, the deferred x += sum alpha_i
 // p_i, the GMRES/GCR solution and direction updates), so the order of the
 // terms, and with it every rounding, is the reference's per-element loop.
-// Each thread walks its elements one at a time; the loads of the next chunk
-// of basis vectors are issued before the current chunk is consumed, which
-// keeps enough bytes in flight to stream the basis at HBM speed despite the
-// chain.
+// Each thread walks its elements two at a time, eight basis vectors' loads of
+// both issued before either chain goes on; a last single element has the next
+// chunk's loads issued before the current chunk is consumed. That keeps enough
+// bytes in flight to stream the basis despite the chains: GMRES(30) at 128^3
+// (k = 1 .. 30, 2.1M rows) 142.5 us per iteration with one element at a time and
+// its next one prefetched into L2, 131.7 with two (one pipelined stream over a
+// resident wave of CTAs: 146).
 // Op concept:
 //   using vt = element type; static constexpr int NB (1 or 2 bases), ND;
 //   long long ld;                               // stride between basis vectors
@@ -113,15 +116,31 @@ __global__ void __launch_bounds__(kThreads) basis_kernel(Op op, long long n, Sto
   for (int b = 0; b < NB; b++) B[b] = op.base(b);
   const long long ld = op.ld;
   const long long estride = (long long)gridDim.x * kThreads;
-  for (long long j = (long long)blockIdx.x * kThreads + threadIdx.x; j < n; j += estride) {
-    // the next element's first chunk heads for L2 while this one runs
-    if (j + estride < n) {
+  long long j = (long long)blockIdx.x * kThreads + threadIdx.x;
+  // two elements at a time, their chunks' loads issued together
+  for (; j + estride < n; j += 2 * estride) {
+    typename Op::St s = op.init(j), z = op.init(j + estride);
+    for (int i0 = 0; i0 < k; i0 += C) {
+      VT p[C][NB], q[C][NB];
 #pragma unroll
       for (int u = 0; u < C; u++)
 #pragma unroll
-        for (int b = 0; b < NB; b++)
-          if (u < k) prefetch_l2(B[b] + (long long)u * ld + j + estride);
+        for (int b = 0; b < NB; b++) {
+          const VT *v = B[b] + (long long)(i0 + u) * ld + j;
+          p[u][b] = i0 + u < k ? v[0] : (VT)0;
+          q[u][b] = i0 + u < k ? v[estride] : (VT)0;
+        }
+#pragma unroll
+      for (int u = 0; u < C; u++)
+        if (i0 + u < k) {
+          op.step(s, i0 + u, p[u]);
+          op.step(z, i0 + u, q[u]);
+        }
     }
+    op.done(j, s, acc);
+    op.done(j + estride, z, acc);
+  }
+  for (; j < n; j += estride) {  // at most one is left
     typename Op::St s = op.init(j);
     VT cur[C][NB], nxt[C][NB];
 #pragma unroll
@@ -500,9 +519,8 @@ inline void launch_vec(ks_ctx *ctx, long long n, const Op &op_in, Stop stop, int
 
 // k_hint: the number of basis vectors, or a bound when the kernel reads it
 // from the device. Short chains run at least one full-occupancy wave of CTAs
-// and at most two elements per thread (measured best at 128^3: fewer CTAs
-// keep the final reduction short, but each element's loads are a round trip
-// the next element waits behind, even with its basis prefetched into L2).
+// and at most two elements per thread, which it works on together (fewer CTAs
+// keep the final reduction short).
 // Long chains (measured: from 64 vectors) stream fastest with one thread per
 // element, the reduction's cost then being small beside the pass.
 template <class Op>

@@ -129,10 +129,12 @@ __global__ void pattern_grad_kernel(CsrK<double> A, const double *__restrict__ l
 // group is the fast grid index (blockIdx.x) and the slice of the vectors the
 // slow one (blockIdx.y): the CTAs of every group that read the same slice of
 // W run together, so W comes from DRAM about once rather than once per group.
-// Each group is reduced deterministically with its own counter;
-// Epi::put(w, i, value) receives every result (thread 0 of the group's last CTA).
+// One left vector: a thread keeps two elements' loads (18 of 8 bytes) in flight
+// in 80 registers, 3 CTAs per SM (one element, 64 registers, 4 CTAs: GMRES(30) at
+// 128^3 5.5 us more per iteration). Each group is reduced deterministically with
+// its own counter; Epi::put(w, i, value) receives every result (thread 0 of the group's last CTA).
 template <int NW, class VT, class Epi>
-__global__ void __launch_bounds__(kThreads, NW == 1 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, NW == 1 ? 3 : 2)
     block_dot_kernel(const VT *__restrict__ V, long long ld, int k,
                      const VT *__restrict__ W0, const VT *__restrict__ W1, long long n,
                      Epi epi, Stop stop, double *partials, unsigned *counters) {
@@ -147,7 +149,29 @@ __global__ void __launch_bounds__(kThreads, NW == 1 ? 4 : 2)
 #pragma unroll
   for (int q = 0; q < NW * G8; q++) acc[q] = 0.0;
   const long long stride = (long long)nslices * kThreads;
-  for (long long j = (long long)slice * kThreads + threadIdx.x; j < n; j += stride) {
+  long long j = (long long)slice * kThreads + threadIdx.x;
+  if constexpr (NW == 1) {
+    // two elements' loads in flight, added one after the other: the order of the
+    // single-element loop below, so the same sums
+    for (; j + stride < n; j += 2 * stride) {
+      const VT wa = W0[j], wb = W0[j + stride];
+      VT va[G8], vb[G8];
+#pragma unroll
+      for (int q = 0; q < G8; q++) {
+        const VT *v = V + (long long)(i0 + q) * ld + j;
+        va[q] = q < cnt ? v[0] : (VT)0;
+        vb[q] = q < cnt ? v[stride] : (VT)0;
+      }
+#pragma unroll
+      for (int q = 0; q < G8; q++) {
+        if (q < cnt) {
+          acc[q] = add_rn(acc[q], mul_rn(widen(wa), widen(va[q])));
+          acc[q] = add_rn(acc[q], mul_rn(widen(wb), widen(vb[q])));
+        }
+      }
+    }
+  }
+  for (; j < n; j += stride) {
     const double w0 = widen(W0[j]);
     const double w1 = NW > 1 ? widen(W1[j]) : 0.0;
 #pragma unroll
