@@ -34,7 +34,11 @@
 // with the iteration's tag in one store (16 bytes in FP64, 8 in FP32): a
 // reader takes a value with its tag and needs no fence and no flag, so the
 // halo arrives in the shadow of the (r, r) reduction. Tags differ from one
-// launch to the next on the same array (ChipArgs::tag0). Element operations
+// launch to the next on the same array (ChipArgs::tag0). With one or two rows per
+// thread r crosses behind a flag per CTA instead, acquired by warp 1 while warp 0
+// waits for the sum (us per iteration, tags / flags: 128^2 3.46 / 3.04, 333^2 4.74 /
+// 4.51; with more rows per thread the flags' kernel spills: 700^2 6.7 / 8.0, 99^3
+// FP32 11.4 / 12.3). Element operations
 // and the order of a row's terms are k_cg_onchip's; only the dot products add
 // their terms in another order. An entry a row does not have is a stored zero
 // and its term a zero added to a sum that starts at +0: no mask is looked at (p
@@ -355,12 +359,17 @@ struct ChipRows<false> {
     n_lo = lo_far + hl2;
     hi_far = hu2 < hu ? min(nr, hu - hu2) : 0;
     n_hi = hi_far + hu2;
+    bl = max(r0 - hl, 0) / a.rpc;
+    nb = min(r0 + nr - 1 + hu, n - 1) / a.rpc - bl + 1;
   }
   __device__ __forceinline__ int pos(int li) const { return hl + li; }
   __device__ __forceinline__ int row(int li) const { return r0 + li; }
   __device__ __forceinline__ bool shared(int li) const { return li < hu || li >= nr - hl; }
   __device__ __forceinline__ int shift(int, int off) const { return off; }
   __device__ __forceinline__ int halo() const { return n_lo + n_hi; }
+  int bl, nb;  // the CTAs that own halo rows
+  __device__ __forceinline__ int ctas() const { return nb; }
+  __device__ __forceinline__ int cta(int i) const { return bl + i == (int)blockIdx.x ? -1 : bl + i; }
   __device__ __forceinline__ void halo_row(int k, int &p, int &g) const {
     int li;
     if (k < n_lo) {
@@ -377,11 +386,12 @@ struct ChipRows<false> {
 
 template <>
 struct ChipRows<true> {
-  int nx, ty, tz, plane, nr, row0, up, pitch;  // up: rows of a plane of the box; pitch: of a plane in shared memory
+  int nx, ty, tz, plane, nr, row0, up, pitch, gy;  // up: rows of a plane of the box; pitch: of a plane in shared memory
   float inv_plane, inv_nx;
   bool y0, y1, z0, z1;  // faces with a neighbour
   __device__ __forceinline__ explicit ChipRows(const ChipArgs &a) {
     const int cy = blockIdx.x % a.gy, cz = blockIdx.x / a.gy;
+    gy = a.gy;
     nx = a.nx;
     ty = min(a.by, a.ny - cy * a.by);
     tz = min(a.bz, a.nz - cz * a.bz);
@@ -410,6 +420,11 @@ struct ChipRows<true> {
     return d < 3 ? -s : s;
   }
   __device__ __forceinline__ int halo() const { return 2 * nx * tz + 2 * plane; }
+  __device__ __forceinline__ int ctas() const { return 4; }
+  __device__ __forceinline__ int cta(int i) const {  // the neighbours (-1: none)
+    const int b = blockIdx.x;
+    return i == 0 ? (y0 ? b - 1 : -1) : i == 1 ? (y1 ? b + 1 : -1) : i == 2 ? (z0 ? b - gy : -1) : (z1 ? b + gy : -1);
+  }
   __device__ __forceinline__ void halo_row(int k, int &p, int &g) const {
     if (k < 2 * plane) {  // z faces: whole planes of the tile
       const bool hi = k >= plane;
@@ -440,6 +455,7 @@ template <class VT, int NDG, int RJ, bool kTile>
 __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_constant__ ChipArgs a) {
   using CV = ChipVals<VT, RJ>;
   constexpr int KD = NDG > 0 ? NDG : kMaxDiag;
+  constexpr bool kFlags = RJ <= 2;  // how r crosses between CTAs
   constexpr bool kXT = (KD + 1) * CV::W <= kChipWords;  // x in TMEM behind the matrix
   static_assert(KD * CV::W <= kChipWords, "the matrix fits a thread's TMEM words");
   static_assert(!kTile || NDG == 7, "tiles are those of a 7-point stencil");
@@ -464,6 +480,10 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
   const int nd = NDG > 0 ? NDG : a.nd;
   const ChipRows<kTile> rows(a);
   const int nr = rows.nr, nh = rows.halo();
+  // the thread's halo rows hk0 + hstep u (flags: none of warp 0, whose hk0 stays
+  // negative for all u)
+  constexpr int hstep = kFlags ? kChipThreads - 32 : kChipThreads;
+  const int hk0 = kFlags ? (t < 32 ? -(1 << 24) : t - 32) : t;
   const bool lead = blockIdx.x == 0 && t == 0;  // keeps the method's state (whole solve)
   // the halo's rows (-1: none) and byte positions, then p with its halo
   int2 *const sh = reinterpret_cast<int2 *>(ir_smem_raw);
@@ -548,7 +568,7 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
     int p, g;
     rows.halo_row(k, p, g);
     p *= (int)sizeof(VT);
-    sh[k] = make_int2(g, p);  // read by the thread that wrote it
+    sh[k] = make_int2(g, p);
     if (g >= 0) P(p) = __ldcg(rin + g);
   }
   tm_wait_st();
@@ -623,11 +643,17 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
         const int li = t + kChipThreads * j;
         if (li < nr) {
           r[j] = add_rn(mul_rn((VT)(-av), q[j]), r[j]);
-          if ((pub >> j) & 1u) chip_pub(a.P, row[j], r[j], tag);
+          if ((pub >> j) & 1u) {
+            if constexpr (kFlags)
+              __stcg((VT *)a.P + row[j], r[j]);
+            else
+              chip_pub(a.P, row[j], r[j], tag);
+          }
           acc = add_rn(acc, mul_rn(widen(r[j]), widen(r[j])));
         }
       }
       chip_post(a, ++gen, acc);
+      if (kFlags && t == 32) st_release_u64(tile_flag(a.sync, blockIdx.x), (unsigned long long)L);
       if constexpr (kXT) {
         VT xv[RJ];
         CV::get(tx, xv);
@@ -640,17 +666,47 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
         for (int j = 0; j < RJ; j++) x[j] = add_rn(mul_rn(av, P(pos[j])), x[j]);
       }
       xw = true;
-      // the halo's r: every row's load issued, then those whose tag is not
-      // this iteration's yet read again (bounded)
+      // the halo's r. Flags: a warp other than the first, which waits for the sum,
+      // acquires the neighbours' and lets the others load. Tags: every row's load
+      // issued, then those whose tag is not this iteration's yet read again
+      // (bounded either way)
       VT h[kChipHalo];
       unsigned late = 0;
+      if constexpr (kFlags) {
+        if (t >= 32) {
+          if (t < 64) {
+            for (int i = t - 32; i < rows.ctas(); i += 32) {
+              const int q = rows.cta(i);
+              ChipClock clk;
+              bool good = true;
+              while (good && q >= 0 && ld_acquire_u64(tile_flag(a.sync, q)) < (unsigned long long)L)
+                good = clk.go_on(a.wait_ns);
+              if (!good) {
+                S.fail = 1;
+                atomicExch(a.err, 1);
+              }
+            }
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(kChipThreads - 32) : "memory");
 #pragma unroll
-      for (int u = 0; u < kChipHalo; u++) {
-        const int k = t + kChipThreads * u;
-        h[u] = (VT)0;
-        if (kChipThreads * u < nh && k < nh) {
-          const int g = sh[k].x;
-          if (g >= 0 && !chip_take(a.P, g, h[u], tag)) late |= 1u << u;
+          for (int u = 0; u < kChipHalo; u++) {
+            const int k = hk0 + hstep * u;
+            h[u] = (VT)0;
+            if (hstep * u < nh && k < nh) {
+              const int g = sh[k].x;
+              if (g >= 0) h[u] = __ldcg((const VT *)a.P + g);
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < kChipHalo; u++) {
+          const int k = hk0 + hstep * u;
+          h[u] = (VT)0;
+          if (hstep * u < nh && k < nh) {
+            const int g = sh[k].x;
+            if (g >= 0 && !chip_take(a.P, g, h[u], tag)) late |= 1u << u;
+          }
         }
       }
       if (late) {
@@ -659,7 +715,7 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
 #pragma unroll
           for (int u = 0; u < kChipHalo; u++)
             if ((late >> u) & 1u)
-              if (chip_take(a.P, sh[t + kChipThreads * u].x, h[u], tag)) late &= ~(1u << u);
+              if (chip_take(a.P, sh[hk0 + hstep * u].x, h[u], tag)) late &= ~(1u << u);
           if (late && !clk.go_on(a.wait_ns)) {
             S.fail = 1;
             atomicExch(a.err, 1);
@@ -690,8 +746,8 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
         if (t + kChipThreads * j < nr) P(pos[j]) = add_rn(mul_rn(bv, P(pos[j])), r[j]);
 #pragma unroll
       for (int u = 0; u < kChipHalo; u++) {
-        const int k = t + kChipThreads * u;
-        if (kChipThreads * u < nh && k < nh) {
+        const int k = hk0 + hstep * u;
+        if (hstep * u < nh && k >= 0 && k < nh) {
           const int2 e = sh[k];
           if (e.x >= 0) P(e.y) = add_rn(mul_rn(bv, P(e.y)), h[u]);
         }
@@ -834,6 +890,7 @@ inline bool chip_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShap
     s->elems = s->hl + (int)rows + s->hu;
   }
   if (halo > kChipHalo * kChipThreads) return false;
+  if (s->rj <= 2 && halo > kChipHalo * (kChipThreads - 32)) return false;
   s->smem = sizeof(VT) * (size_t)s->elems + sizeof(int2) * (size_t)halo;
   return s->smem + 2048 <= (size_t)optin;  // + the static arrays
 }
