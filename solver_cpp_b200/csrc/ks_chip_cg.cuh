@@ -36,8 +36,8 @@
 // halo arrives in the shadow of the (r, r) reduction. Tags differ from one
 // launch to the next on the same array (ChipArgs::tag0). With one or two rows per
 // thread r crosses behind a flag per CTA instead, acquired by warp 1 while warp 0
-// waits for the sum (us per iteration, tags / flags: 128^2 3.46 / 3.04, 333^2 4.74 /
-// 4.51; with more rows per thread the flags' kernel spills: 700^2 6.7 / 8.0, 99^3
+// waits for the sum (us per iteration, tags / flags: 128^2 3.46 / 3.10, 333^2 4.74 /
+// 4.56; with more rows per thread the flags' kernel spills: 700^2 6.7 / 8.0, 99^3
 // FP32 11.4 / 12.3). Element operations
 // and the order of a row's terms are k_cg_onchip's; only the dot products add
 // their terms in another order. An entry a row does not have is a stored zero
@@ -46,9 +46,9 @@
 // outside the matrix has p = 0.
 //
 // What bounds an iteration: latency, the two grid reductions before all (1.2
-// to 1.6 us each; 333^2: of 4.7 us per iteration about 3.3). Measured, us per
+// to 1.6 us each; 333^2: of 4.6 us per iteration about 3.3). Measured, us per
 // iteration, k_cg_onchip or the kernel it replaces / k_cg_chip: FP64 CG 128^2
-// 4.39 / 3.46, 333^2 14.5 / 4.73, 512^2 11.8 / 5.11, 64^3 13.3 / 5.8, 81^3 17.5
+// 4.39 / 3.10, 333^2 14.5 / 4.56, 512^2 11.8 / 5.11, 64^3 13.3 / 5.8, 81^3 17.5
 // / 8.0; FP32 inner CG 24^3 17.9 / 3.8, 64^3 13.3 / 5.7, 99^3 (BF16 values)
 // 18.3 / 11.4. The largest systems are bound by the instructions per row (7
 // products from shared memory, FP64 sums of FP32 rows).
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(kChipThreads, 1) k_cg_chip(const __grid_consta
 // grid reductions poll their slots directly and are 0.3-0.4 us cheaper each:
 // 512 rows per CTA until that many are in use, then more rows on the same
 // number up to 2,048 (65,536 rows), then one CTA per SM. Measured, us per CG
-// iteration (FP64): 112^2 on 13 / 25 / 49 CTAs 3.57 / 3.39 / 4.17, 150^2 on 22
+// iteration (FP64, r always with tags): 112^2 on 13 / 25 / 49 CTAs 3.57 / 3.39 / 4.17, 150^2 on 22
 // / 30 / 44 3.52 / 3.52 / 4.30, 256^2 on 32 / 64 / 128 3.91 / 4.51 / 4.29,
 // 333^2 on 55 / 109 / 148 5.07 / 4.66 / 4.72.
 inline long long chip_ctas(long long n, long long sms) {
