@@ -357,13 +357,18 @@ __global__ void __launch_bounds__(kChipThreads, 1)
       for (int c = 0; c < rows.blocks; c++) {
         const TileBlock k(rows, c);
         double *pp = sp + k.pos;
-        double r[C];
+        double r[C], p[C];
         CV::get(tr + CV::W * c, r);
+        // planes past the tile's last one read that one, as in A: p holds one plane
+        // behind it, and a block reaches up to seven
 #pragma unroll
-        for (int u = 0; u < C; u++) {
-          const double w = add_rn(mul_rn(bv, pp[u * sc]), r[u]);
-          if (k.in && k.z0 + u < rows.tz) pp[u * sc] = w;
+        for (int u = 0, o = 0; u < C; u++) {
+          p[u] = pp[o];
+          o += k.z0 + u + 1 < rows.tz ? sc : 0;
         }
+#pragma unroll
+        for (int u = 0; u < C; u++)
+          if (k.in && k.z0 + u < rows.tz) pp[u * sc] = add_rn(mul_rn(bv, p[u]), r[u]);
       }
       if (t >= 32) {
         halo_z(t - 32, kTileHaloThreads, [&](int u, int side, int p, int) { sp[p] = add_rn(mul_rn(bv, sp[p]), hz[u][side]); });

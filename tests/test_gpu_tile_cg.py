@@ -1,0 +1,57 @@
+"""GPU: k_cg_tile (ks_tile_cg.cuh), CG of constant-coefficient boxes on tiles of
+lines, against the kernel-per-step engine.
+
+Element operations are the engine's and only the dot products add their terms in
+another order. The systems are diagonally dominant by 5 %, so the histories and
+solutions of the first iterations agree to 1e-9 (as in test_gpu_chip_cg.py).
+
+Which tile a box gets: by lines and bz planes as named below (148 SMs, 227 KB of
+shared memory per CTA). A thread works on blocks of 8 planes, so what can go
+wrong lies at bz mod 8, at last tiles thinner than the others, and at boxes that
+are one tile high or deep.
+"""
+import numpy as np
+import pytest
+
+from solver_cpp_b200.matrices import poisson3d
+from test_gpu_chip_cg import agree, both
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (67, 56, 162),    # by 7, bz 9: a block of one plane
+    (46, 14, 1261),   # bz 18, the last tile one plane
+    (113, 113, 113),  # bz 11, the last tile 3 planes
+    (315, 241, 8),    # by 4, the last one line; bz 4: less than a block
+    (117, 117, 117),  # bz 13
+    (124, 124, 124),  # bz 14
+    (21, 111, 261),   # bz 15
+    (9, 300, 301),    # by 43; the last tile one plane
+    (311, 3, 784),    # one tile in y
+    (158, 1284, 3),   # one tile in z, of three planes
+    (3, 848, 924),    # by 170, bz 32: 2.35M rows
+]
+
+
+def constant_box(shape, skew=0.0):
+    """-1 beside a dominant diagonal; with skew every diagonal has a value of its own."""
+    A = poisson3d(*shape)
+    off = A.col - np.repeat(np.arange(A.n), np.diff(A.ptr))
+    for k, o in enumerate(np.unique(off)):
+        A.val[off == o] = 6.3 if o == 0 else -1.0 + skew * (k - 3)
+    return A
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_against_engine(ks, ctx, shape):
+    chip, step = both(ks, ctx, constant_box(shape), L=30)
+    assert chip.report["n_mv"] == 1 and chip.report["n_dot"] == 0, chip.report
+    agree(chip, step)
+
+
+@pytest.mark.parametrize("shape", [(93, 91, 90), (113, 113, 113), (131, 62, 77)])
+def test_unsymmetric_constants(ks, ctx, shape):
+    """Seven different values, A not its transpose: each neighbour takes its own."""
+    chip, step = both(ks, ctx, constant_box(shape, skew=0.01), L=15)
+    assert chip.report["n_mv"] == 1 and chip.report["n_dot"] == 0, chip.report
+    agree(chip, step)
