@@ -10,7 +10,7 @@ namespace ks {
 template <class... KArgs, class... Args>
 static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShape &sh, bool probe, bool *fits, int cls,
                                int threads, const Args &...args) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  cudaError_t e = allow_smem(ctx, fn);
   if (e != cudaSuccess) return e;
   if (probe) {
     int b = 0;

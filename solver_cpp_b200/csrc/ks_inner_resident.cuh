@@ -74,6 +74,23 @@ inline size_t ir_sync_bytes(int G) {
          (2 * sizeof(ulonglong2) + 32) * (size_t)G;
 }
 
+// Lets a kernel be launched with as much dynamic shared memory as a CTA can have
+// beside the kernel's static arrays. The limit belongs to the kernel and the
+// device, not to a context: were it set to the size of one launch, a thread with
+// a smaller system could lower it between another thread's call and its launch,
+// which then fails.
+template <class... KArgs>
+inline cudaError_t allow_smem(const ks_ctx *ctx, void (*fn)(KArgs...)) {
+  int optin = 0;
+  cudaFuncAttributes at{};
+  cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
+  const int room = optin - (int)at.sharedSizeBytes;
+  if (e == cudaSuccess && at.maxDynamicSharedSizeBytes != room)
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+  return e;
+}
+
 struct IrArgs {
   const void *rin;  // inner solve: r rounded to FP32; whole solve: b (FP64); n entries
   void *x;          // the solution (the kernel's precision), n
@@ -1294,7 +1311,7 @@ template <int NDG, bool kC>
 inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, const IrArgs &a, size_t smem,
                                int G, bool probe, bool *fits) {
   auto fn = k_bicg_onchip<NDG, kC>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(ctx, fn);
   if (e != cudaSuccess) return e;
   if (probe) {
     int b = 0;
@@ -1683,7 +1700,7 @@ template <class VT, class MT, int NDG, bool kC>
 inline cudaError_t ir_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
                                bool *fits, int cls) {
   auto fn = k_cg_onchip<VT, MT, NDG, kC>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  cudaError_t e = allow_smem(ctx, fn);
   if (e != cudaSuccess) return e;
   if (probe) {
     int b = 0;
@@ -1727,7 +1744,7 @@ template <int NDG, bool kC>
 inline cudaError_t icr_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, const IrShape &sh, bool probe,
                                 bool *fits) {
   auto fn = k_cr_onchip<NDG, kC>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+  cudaError_t e = allow_smem(ctx, fn);
   if (e != cudaSuccess) return e;
   if (probe) {
     int b = 0;
