@@ -80,6 +80,10 @@ const char *ks_status_string(ks_status s);
  * `times` class counts time, not launches: times.hpp:15-88). */
 int64_t ks_ctx_launches(const ks_ctx *ctx);
 const char *ks_last_error(const ks_ctx *ctx);
+/* Name of the kernel that ran the context's last solve (a VP method: its inner
+ * solves) in one launch, as k_cg_tile; "" where there was one kernel per step.
+ * Valid until the context's next solve. No counterpart in the reference. */
+const char *ks_ctx_solve_kernel(const ks_ctx *ctx);
 int ks_abi_version(void);
 /* Limit of every bounded device wait of this context's kernels (the SpMV's
  * shared-memory staging barriers), in nanoseconds; ns <= 0 restores the

@@ -88,6 +88,11 @@ class Context:
         """Limit of the kernels' bounded device waits in ns (<= 0: the 2 s default)."""
         _check(lib().ks_ctx_set_wait_limit(self.handle, int(ns)), self.handle, "set_wait_limit")
 
+    def solve_kernel(self) -> str:
+        """The kernel that ran the last solve (a VP method: its inner solves) in
+        one launch; "" where there was one kernel per step."""
+        return lib().ks_ctx_solve_kernel(self.handle).decode()
+
     def matrix(self, A: CSR, transpose=False, fp32=False, bf16=False, index32=False, diag=True) -> "Matrix":
         return Matrix(self, A, transpose=transpose, fp32=fp32, bf16=bf16, index32=index32, diag=diag)
 

@@ -89,6 +89,7 @@ SIGNATURES = [
     ("ks_status_string", C.c_char_p, [C.c_int]),
     ("ks_ctx_launches", C.c_int64, [_VP]),
     ("ks_last_error", C.c_char_p, [_VP]),
+    ("ks_ctx_solve_kernel", C.c_char_p, [_VP]),
     ("ks_abi_version", C.c_int, []),
     ("ks_ctx_set_wait_limit", C.c_int, [_VP, C.c_int64]),
     ("ks_csr_upload", C.c_int, [_VP, _I64, _I64, _VP, _VP, _VP, C.c_uint, C.POINTER(_VP)]),

@@ -5,11 +5,11 @@
 
 namespace ks {
 
-// A cooperative launch of fn(args...), or with `probe` only the check that it
-// can be co-resident.
+// A cooperative launch of fn(args...), the kernel `name`, or with `probe` only
+// the check that it can be co-resident.
 template <class... KArgs, class... Args>
-static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShape &sh, bool probe, bool *fits, int cls,
-                               int threads, const Args &...args) {
+static cudaError_t coop_launch(ks_ctx *ctx, const char *name, void (*fn)(KArgs...), const ChipShape &sh, bool probe,
+                               bool *fits, int cls, int threads, const Args &...args) {
   cudaError_t e = allow_smem(ctx, fn);
   if (e != cudaSuccess) return e;
   if (probe) {
@@ -28,6 +28,7 @@ static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShap
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  ctx->solve_kernel = name;
   ctx->launches++;
   ProfLaunch pl(ctx, cls);
   return cudaLaunchKernelEx(&cfg, fn, args...);
@@ -35,7 +36,7 @@ static cudaError_t coop_launch(ks_ctx *ctx, void (*fn)(KArgs...), const ChipShap
 
 template <class VT, int NDG, int RJ, bool kTile>
 static cudaError_t chip_launch_n(ks_ctx *ctx, const ChipArgs &a, const ChipShape &sh, bool probe, bool *fits, int cls) {
-  return coop_launch(ctx, k_cg_chip<VT, NDG, RJ, kTile>, sh, probe, fits, cls, kChipThreads, a);
+  return coop_launch(ctx, "k_cg_chip", k_cg_chip<VT, NDG, RJ, kTile>, sh, probe, fits, cls, kChipThreads, a);
 }
 
 template <class VT, int NDG, bool kTile>
@@ -66,11 +67,11 @@ cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const C
                         int cls) {
   TileDiag D{};
   for (int k = 0; k < 7; k++) D.v[k] = A.dia_cv[k];
-  return coop_launch(ctx, k_cg_tile, sh, probe, fits, cls, kChipThreads, a, D);
+  return coop_launch(ctx, "k_cg_tile", k_cg_tile, sh, probe, fits, cls, kChipThreads, a, D);
 }
 
 cudaError_t csr_launch(ks_ctx *ctx, const CsrCgArgs &a, const CsrShape &sh, bool probe, bool *fits, int cls) {
-  auto run = [&](auto kern) { return coop_launch(ctx, kern, sh, probe, fits, cls, sh.threads, a); };
+  auto run = [&](auto kern) { return coop_launch(ctx, "k_cg_csr", kern, sh, probe, fits, cls, sh.threads, a); };
   if (sh.threads == 1024) return run(k_cg_csr<1024, 4>);  // more than 2,048 rows per CTA
   return sh.rj == 1 ? run(k_cg_csr<512, 1>) : sh.rj == 2 ? run(k_cg_csr<512, 2>) : run(k_cg_csr<512, 4>);
 }

@@ -330,6 +330,7 @@ struct ks_ctx {
   std::vector<bool> pool_busy;
   std::string last_error;
   long long launches = 0;       // kernels launched (diagnostics)
+  const char *solve_kernel = "";  // the one-launch kernel of the last solve (ks_ctx_solve_kernel)
   // Row-split solve in progress: its communicator (reductions are summed over
   // the ranks), the first transport error, the stage of the summed values,
   // and the outer method's `done` with a mapped snapshot ring for polling.

@@ -821,6 +821,8 @@ const char *ks_status_string(ks_status s) {
 
 const char *ks_last_error(const ks_ctx *ctx) { return ctx ? ctx->last_error.c_str() : ""; }
 
+const char *ks_ctx_solve_kernel(const ks_ctx *ctx) { return ctx ? ctx->solve_kernel : ""; }
+
 int64_t ks_ctx_launches(const ks_ctx *ctx) { return ctx ? ctx->launches : 0; }
 
 ks_status ks_ctx_create(int device, ks_ctx **out) {

@@ -1329,6 +1329,7 @@ inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, co
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  ctx->solve_kernel = "k_bicg_onchip";
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, kMv);  // a profiled solve counts the whole solve as one SpMV-class launch
@@ -1718,6 +1719,7 @@ inline cudaError_t ir_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, co
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  ctx->solve_kernel = "k_cg_onchip";
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, cls);
@@ -1762,6 +1764,7 @@ inline cudaError_t icr_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, c
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  ctx->solve_kernel = "k_cr_onchip";
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, kMv);  // a profiled solve counts the whole solve as one SpMV-class launch

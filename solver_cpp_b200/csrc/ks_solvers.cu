@@ -795,6 +795,7 @@ inline bool run_cg_resident(const Env<double> &E, const double *b, double *x, ks
   launch_scalar(E.ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
   E.ctx->launches++;
   ProfLaunch pl(E.ctx, kOther);  // a whole solve in one cluster launch
+  E.ctx->solve_kernel = "k_cg_resident";
   const cudaError_t e = res_cg(sh, A.col16 != nullptr, E.ctx->stream, a, false, nullptr);
   *s = e == cudaSuccess ? KS_OK : cuda_fail(E.ctx, e, "cluster-resident CG launch");
   return true;
@@ -1032,6 +1033,7 @@ inline bool run_cr_resident(const Env<double> &E, const double *b, double *x, ks
   launch_scalar(E.ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
   E.ctx->launches++;
   ProfLaunch pl(E.ctx, kOther);  // a whole solve in one cluster launch
+  E.ctx->solve_kernel = "k_cr_resident";
   const cudaError_t e = res_cr(sh, A.col16 != nullptr, E.ctx->stream, a, false, nullptr);
   *s = e == cudaSuccess ? KS_OK : cuda_fail(E.ctx, e, "cluster-resident CR launch");
   return true;
@@ -1335,6 +1337,7 @@ inline bool run_bicg_resident(const Env<double> &E, const double *b, double *x, 
   launch_scalar(E.ctx, InitOp{E.st, E.sp.eps, E.sp.maxloop, E.record ? 1 : 0}, Stop{nullptr, E.outer_done});
   E.ctx->launches++;
   ProfLaunch pl(E.ctx, kOther);  // a whole solve in one cluster launch
+  E.ctx->solve_kernel = "k_bicg_resident";
   const cudaError_t e = res_bicg(sh, ia16, it16, E.ctx->stream, a, false, nullptr);
   *s = e == cudaSuccess ? KS_OK : cuda_fail(E.ctx, e, "cluster-resident BiCG launch");
   return true;
@@ -2796,6 +2799,7 @@ using namespace ks;
 static ks_status solve_impl(ks_ctx *ctx, const ks_mat *mat, ks_solver outer, ks_solver inner,
                             const ks_params *prm, const double *b, double *x, int64_t *hist_iter,
                             double *hist_err, int64_t hist_cap, ks_report *rep) {
+  ctx->solve_kernel = "";
   if (outer == KS_KSKIPCR || outer == KS_VPBICG)
     return set_error(ctx, KS_UNIMPLEMENTED, "Not implemented (as in the reference)");
   const bool vp = is_vp(outer);

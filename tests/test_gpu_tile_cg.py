@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 
 from solver_cpp_b200.matrices import poisson3d
-from test_gpu_chip_cg import agree, both
+from test_gpu_chip_cg import agree
 
 pytestmark = pytest.mark.gpu
 
@@ -42,16 +42,35 @@ def constant_box(shape, skew=0.0):
     return A
 
 
+def both(ks, ctx, A, b=None, **kw):
+    """The solve on tiles and kernel by kernel."""
+    M = ctx.matrix(A)
+    b = np.random.default_rng(1).standard_normal(A.n) if b is None else b
+    tile = ks.solve(ctx, M, "CG", b, cluster_solve=0, **kw)
+    assert ctx.solve_kernel() == "k_cg_tile"
+    step = ks.solve(ctx, M, "CG", b, cluster_solve=1, **kw)
+    assert ctx.solve_kernel() == ""
+    M.close()
+    return tile, step
+
+
 @pytest.mark.parametrize("shape", SHAPES)
 def test_against_engine(ks, ctx, shape):
-    chip, step = both(ks, ctx, constant_box(shape), L=30)
-    assert chip.report["n_mv"] == 1 and chip.report["n_dot"] == 0, chip.report
-    agree(chip, step)
+    agree(*both(ks, ctx, constant_box(shape), E=1e-14, L=30))
 
 
 @pytest.mark.parametrize("shape", [(93, 91, 90), (113, 113, 113), (131, 62, 77)])
 def test_unsymmetric_constants(ks, ctx, shape):
     """Seven different values, A not its transpose: each neighbour takes its own."""
-    chip, step = both(ks, ctx, constant_box(shape, skew=0.01), L=15)
-    assert chip.report["n_mv"] == 1 and chip.report["n_dot"] == 0, chip.report
-    agree(chip, step)
+    agree(*both(ks, ctx, constant_box(shape, skew=0.01), E=1e-14, L=15))
+
+
+@pytest.mark.parametrize("L", [0, 1, 2])
+def test_stops_at_maxloop(ks, ctx, L):
+    agree(*both(ks, ctx, constant_box((93, 91, 90)), E=1e-14, L=L))
+
+
+def test_converges(ks, ctx):
+    tile, step = both(ks, ctx, constant_box((113, 113, 113)), E=1e-9)
+    assert tile.converged and tile.true_rel_res < 2e-9
+    agree(tile, step)
