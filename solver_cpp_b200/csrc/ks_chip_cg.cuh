@@ -54,6 +54,8 @@
 // products from shared memory, FP64 sums of FP32 rows).
 #pragma once
 
+#include <cmath>
+
 #include "ks_inner_resident.cuh"
 
 namespace ks {
@@ -938,10 +940,14 @@ constexpr int kTileHaloThreads = kChipThreads - 32;  // warps 1 .. 15
 constexpr int kTileHaloZ = 3, kTileHaloY = 4;  // columns of a z face, rows of a y face per thread of them at most
 
 // The tile with the least work (the rows its threads walk, plus half a row for
-// each of the halo's) on at most one CTA per SM; false where none fits on chip.
+// each of the halo's) on at most one CTA per SM; false where none fits on chip or a
+// value is not finite.
 inline bool tile_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShape *s) {
   const long long sms = std::min(ctx->num_sms, (int)kChipMaxGrid);
   if (A.dia_box < 2 || !A.dia_cst || A.dia_cmin != 0 || A.dia_cmax != n || n > sms * kTileRows * kChipThreads) return false;
+  // an absent entry's term is its diagonal's value times a zero: NaN where the value is not finite
+  for (int k = 0; k < 7; k++)
+    if (!std::isfinite(A.dia_cv[k])) return false;
   int optin = 0;
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
     (void)cudaGetLastError();

@@ -74,3 +74,18 @@ def test_converges(ks, ctx):
     tile, step = both(ks, ctx, constant_box((113, 113, 113)), E=1e-9)
     assert tile.converged and tile.true_rel_res < 2e-9
     agree(tile, step)
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("diagonal", [0, 5])
+def test_constants_that_are_not_finite(ks, ctx, value, diagonal):
+    """An entry a row does not have must not count: inf times the zero beside the
+    box would be NaN."""
+    A = constant_box((93, 91, 90))
+    off = A.col - np.repeat(np.arange(A.n), np.diff(A.ptr))
+    A.val[off == np.unique(off)[diagonal]] = -value
+    M = ctx.matrix(A)
+    chip, step = [ks.solve(ctx, M, "CG", np.ones(A.n), E=1e-14, L=10, cluster_solve=c) for c in (0, 1)]
+    M.close()
+    assert chip.status == step.status and chip.loop == step.loop, (chip.status, step.status, chip.loop, step.loop)
+    assert np.array_equal(chip.hist_err, step.hist_err, equal_nan=True)
