@@ -95,8 +95,17 @@ extern "C" ks_status ks_block_dot_noalloc(const double *V, int64_t ld, int k, co
   long long gx = (n + kThreads - 1) / kThreads;
   if (gx > kNoAllocGrid) gx = kNoAllocGrid;
   dim3 grid((unsigned)groups, (unsigned)gx);
-  block_dot_kernel<1, double, PutArray><<<grid, kThreads, 0, st>>>(V, ld, k, w, nullptr, n, PutArray{h, 0, 1},
-                                                                  Stop{nullptr, nullptr}, partials, counters);
+  auto run = [&](auto kern) {
+    kern<<<grid, kThreads, 0, st>>>(V, ld, k, w, nullptr, n, PutArray{h, 0, 1}, Stop{nullptr, nullptr}, partials, counters);
+  };
+  // Two elements at a time where the vectors come from memory (L2 holds 126 MB),
+  // but for two groups: those fill the GPU in one wave of one element's 4 CTAs per
+  // SM, and not of two elements' 3. us, one element / two: 2.1M rows 4 vectors 22.2
+  // / 24.6, 8 43 / 33, 16 52 / 60, 24 84 / 72, 64 183 / 179; 303K rows 24 16.5 / 17.5.
+  if (groups != 2 && 8LL * (k + 1) * n > 120000000)
+    run(block_dot_kernel<1, double, PutArray, true>);
+  else
+    run(block_dot_kernel<1, double, PutArray>);
   e = cudaGetLastError();
   return e == cudaSuccess ? KS_OK : KS_CUDA_ERROR;
 }

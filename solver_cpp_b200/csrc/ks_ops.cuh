@@ -129,12 +129,13 @@ __global__ void pattern_grad_kernel(CsrK<double> A, const double *__restrict__ l
 // group is the fast grid index (blockIdx.x) and the slice of the vectors the
 // slow one (blockIdx.y): the CTAs of every group that read the same slice of
 // W run together, so W comes from DRAM about once rather than once per group.
-// One left vector: a thread keeps two elements' loads (18 of 8 bytes) in flight
-// in 80 registers, 3 CTAs per SM (one element, 64 registers, 4 CTAs: GMRES(30) at
-// 128^3 5.5 us more per iteration). Each group is reduced deterministically with
-// its own counter; Epi::put(w, i, value) receives every result (thread 0 of the group's last CTA).
-template <int NW, class VT, class Epi>
-__global__ void __launch_bounds__(kThreads, NW == 1 ? 3 : 2)
+// Each group is reduced deterministically with its own counter; Epi::put(w, i,
+// value) receives every result (thread 0 of the group's last CTA).
+// kPair (one FP64 left vector): a thread keeps two elements' loads (18 of 8 bytes) in
+// flight in 80 registers, 3 CTAs per SM; otherwise one element's, in 64, 4 CTAs,
+// so that the red_grid slices of one group run in one wave (block_dot_pair).
+template <int NW, class VT, class Epi, bool kPair = false>
+__global__ void __launch_bounds__(kThreads, NW == 1 ? (kPair ? 3 : 4) : 2)
     block_dot_kernel(const VT *__restrict__ V, long long ld, int k,
                      const VT *__restrict__ W0, const VT *__restrict__ W1, long long n,
                      Epi epi, Stop stop, double *partials, unsigned *counters) {
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, NW == 1 ? 3 : 2)
   for (int q = 0; q < NW * G8; q++) acc[q] = 0.0;
   const long long stride = (long long)nslices * kThreads;
   long long j = (long long)slice * kThreads + threadIdx.x;
-  if constexpr (NW == 1) {
+  if constexpr (NW == 1 && kPair) {
     // two elements' loads in flight, added one after the other: the order of the
     // single-element loop below, so the same sums
     for (; j + stride < n; j += 2 * stride) {
@@ -186,9 +187,15 @@ __global__ void __launch_bounds__(kThreads, NW == 1 ? 3 : 2)
   pdl_trigger();
   double *part = partials + (size_t)g * NW * G8 * nslices;
   if (grid_sum_n<NW * G8>(acc, part, counters + g, nslices, slice) && threadIdx.x == 0) {
+    // through shared memory: held in registers they are saved around each call
+    // that an epilogue makes (GCR's divisions: 350 bytes)
+    __shared__ double sums[NW * G8];
+#pragma unroll
+    for (int q = 0; q < NW * G8; q++) sums[q] = acc[q];
+#pragma unroll 1
     for (int q = 0; q < cnt; q++) {
-      epi.put(0, i0 + q, acc[q]);
-      if (NW > 1) epi.put(1, i0 + q, acc[G8 + q]);
+      epi.put(0, i0 + q, sums[q]);
+      if (NW > 1) epi.put(1, i0 + q, sums[G8 + q]);
     }
   }
 }
@@ -220,6 +227,19 @@ struct PutSummed {
   }
 };
 
+// Whether the block dot works on two elements at a time: where the vectors come
+// from memory (L2 holds 126 MB), a thread has four elements at least and three
+// groups or more fill several waves; otherwise the fourth CTA of an SM does more.
+// Measured in Arnoldi steps (FP64, us per dot, one element / two): 150K rows 61..200
+// vectors 64 / 76, 303K 25..30 24.6 / 26.7, 606K 1..8 14.8 / 17.2, 25..30 41.3 /
+// 39.6, 31..60 59 / 56, 1M 1..8 16.6 / 20.5, 9..16 30.6 / 31.7, 17..24 45.1 / 44.0,
+// 2.1M 1..8 29.3 / 33.1, 9..16 55.4 / 54.5, 17..24 77.5 / 74.8, 31..60 148 / 141.
+// FP64 only: of FP32 vectors (an inner GMRES, 40 steps at 160^3) the dots take 9.7
+// ms one element at a time and 21.3 two at a time.
+inline bool block_dot_pair(int k, long long n) {
+  return k > 2 * kBlockDotGroup && n >= 606208 && 8LL * k * n > 120000000;
+}
+
 template <int NW, class VT, class Epi>
 inline ks_status launch_block_dot(ks_ctx *ctx, const VT *V, long long ld, int k, const VT *W0,
                                   const VT *W1, long long n, const Epi &epi, Stop stop) {
@@ -231,18 +251,25 @@ inline ks_status launch_block_dot(ks_ctx *ctx, const VT *V, long long ld, int k,
   const long long need = (n + kThreads - 1) / kThreads;
   if (need < gx) gx = (int)std::max<long long>(need, 1);
   dim3 grid(groups, gx);
+  auto run = [&](const auto &e) {
+    using E = std::decay_t<decltype(e)>;
+    auto go = [&](auto kern) {
+      ctx->next_class = kDot;
+      launch_k(ctx, kern, grid, dim3(kThreads), 0, V, ld, k, W0, W1, n, e, stop, ctx->partials, ctx->counters + 16);
+    };
+    if constexpr (NW == 1 && std::is_same<VT, double>::value) {
+      if (block_dot_pair(k, n)) return go(block_dot_kernel<1, VT, E, true>);
+    }
+    go(block_dot_kernel<NW, VT, E>);
+  };
   if (ctx->red_comm) {  // split solve: results summed over the ranks, then put
     if (NW * k > kStageLen) return set_error(ctx, KS_BAD_INPUT, "block dot: too many results for a split solve");
-    ctx->next_class = kDot;
-    launch_k(ctx, block_dot_kernel<NW, VT, StagePuts<Epi>>, grid, dim3(kThreads), 0, V, ld, k, W0, W1, n,
-             StagePuts<Epi>{ctx->d_stage, k}, stop, ctx->partials, ctx->counters + 16);
+    run(StagePuts<Epi>{ctx->d_stage, k});
     note_dist(ctx, ctx->red_comm->allreduce(ctx->d_stage, NW * k));
     launch_scalar(ctx, PutSummed<Epi>{epi, ctx->d_stage, NW, k}, stop);
     return KS_OK;
   }
-  ctx->next_class = kDot;
-  launch_k(ctx, block_dot_kernel<NW, VT, Epi>, grid, dim3(kThreads), 0, V, ld, k, W0, W1, n, epi, stop,
-           ctx->partials, ctx->counters + 16);
+  run(epi);
   return KS_OK;
 }
 
