@@ -182,9 +182,6 @@ __device__ __forceinline__ float mval<float, __nv_bfloat16>(__nv_bfloat16 v) {
   return __bfloat162float(v);
 }
 
-// Hint: bring the line holding p into L2 (no register, no fault on use).
-__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // ---------------------------------------------------------------- PDL
 // Programmatic dependent launch: every kernel lets the next one in the stream
 // be scheduled at once (trigger) and waits for the previous one's results

@@ -94,14 +94,22 @@ __global__ void __launch_bounds__(kThreads)
 //   static constexpr bool kFinishOnly;          // ND == 0 and finish() still runs
 // Loads in flight per element: kBasisLoads (split over the NB bases).
 constexpr int kBasisLoads = 8;
+constexpr int kBasisOneCtas = 4;  // CTAs per SM of the one-element kernel
 
 template <class Op, class = void>
 struct finish_only : std::false_type {};
 template <class Op>
 struct finish_only<Op, std::void_t<decltype(Op::kFinishOnly)>> : std::integral_constant<bool, Op::kFinishOnly> {};
 
-template <class Op>
-__global__ void __launch_bounds__(kThreads) basis_kernel(Op op, long long n, Stop stop, Red red) {
+// kOne (launch_basis): no thread has more than one element and the CTAs, 4 per
+// SM, run in one wave. Without a loop over elements the compiler keeps a chunk's
+// loads in up to 64 registers (in 40 otherwise, with 6 CTAs per SM). us per block
+// AXPY, in the loop / without: 10K rows 64 vectors 9.3 / 8.2, 300 31.8 / 26.8; 150K
+// rows 30 vectors 10.3 / 9.5, 300 70.3 / 62.4. With more CTAs than one wave of 4
+// per SM it is the slower one (200K rows, 300 vectors 82 / 102).
+template <class Op, bool kOne>
+__global__ void __launch_bounds__(kThreads, kOne ? kBasisOneCtas : 0)
+    basis_kernel(Op op, long long n, Stop stop, Red red) {
   using VT = typename Op::vt;
   constexpr int NB = Op::NB, C = kBasisLoads / NB;
   constexpr int ND = Op::ND > 0 ? Op::ND : 1;
@@ -117,30 +125,7 @@ __global__ void __launch_bounds__(kThreads) basis_kernel(Op op, long long n, Sto
   const long long ld = op.ld;
   const long long estride = (long long)gridDim.x * kThreads;
   long long j = (long long)blockIdx.x * kThreads + threadIdx.x;
-  // two elements at a time, their chunks' loads issued together
-  for (; j + estride < n; j += 2 * estride) {
-    typename Op::St s = op.init(j), z = op.init(j + estride);
-    for (int i0 = 0; i0 < k; i0 += C) {
-      VT p[C][NB], q[C][NB];
-#pragma unroll
-      for (int u = 0; u < C; u++)
-#pragma unroll
-        for (int b = 0; b < NB; b++) {
-          const VT *v = B[b] + (long long)(i0 + u) * ld + j;
-          p[u][b] = i0 + u < k ? v[0] : (VT)0;
-          q[u][b] = i0 + u < k ? v[estride] : (VT)0;
-        }
-#pragma unroll
-      for (int u = 0; u < C; u++)
-        if (i0 + u < k) {
-          op.step(s, i0 + u, p[u]);
-          op.step(z, i0 + u, q[u]);
-        }
-    }
-    op.done(j, s, acc);
-    op.done(j + estride, z, acc);
-  }
-  for (; j < n; j += estride) {  // at most one is left
+  auto one = [&]() {
     typename Op::St s = op.init(j);
     VT cur[C][NB], nxt[C][NB];
 #pragma unroll
@@ -162,6 +147,34 @@ __global__ void __launch_bounds__(kThreads) basis_kernel(Op op, long long n, Sto
         for (int b = 0; b < NB; b++) cur[u][b] = nxt[u][b];
     }
     op.done(j, s, acc);
+  };
+  if constexpr (kOne) {
+    if (j < n) one();
+  } else {
+    // two elements at a time, their chunks' loads issued together
+    for (; j + estride < n; j += 2 * estride) {
+      typename Op::St s = op.init(j), z = op.init(j + estride);
+      for (int i0 = 0; i0 < k; i0 += C) {
+        VT p[C][NB], q[C][NB];
+#pragma unroll
+        for (int u = 0; u < C; u++)
+#pragma unroll
+          for (int b = 0; b < NB; b++) {
+            const VT *v = B[b] + (long long)(i0 + u) * ld + j;
+            p[u][b] = i0 + u < k ? v[0] : (VT)0;
+            q[u][b] = i0 + u < k ? v[estride] : (VT)0;
+          }
+#pragma unroll
+        for (int u = 0; u < C; u++)
+          if (i0 + u < k) {
+            op.step(s, i0 + u, p[u]);
+            op.step(z, i0 + u, q[u]);
+          }
+      }
+      op.done(j, s, acc);
+      op.done(j + estride, z, acc);
+    }
+    for (; j < n; j += estride) one();  // at most one is left
   }
   pdl_trigger();
   if constexpr (Op::ND > 0) {
@@ -531,7 +544,10 @@ inline void launch_basis(ks_ctx *ctx, long long n, int k_hint, const Op &op, Sto
   grid = std::max(1LL, std::min(grid, cap));
   with_rank_sums(ctx, op, stop, [&](const auto &o) {
     using O = std::decay_t<decltype(o)>;
-    launch_k(ctx, basis_kernel<O>, dim3((unsigned)grid), dim3(kThreads), 0, o, n, stop, red_of(ctx, slot));
+    if (grid * kThreads >= n && grid <= (long long)kBasisOneCtas * ctx->num_sms)
+      launch_k(ctx, basis_kernel<O, true>, dim3((unsigned)grid), dim3(kThreads), 0, o, n, stop, red_of(ctx, slot));
+    else
+      launch_k(ctx, basis_kernel<O, false>, dim3((unsigned)grid), dim3(kThreads), 0, o, n, stop, red_of(ctx, slot));
   });
 }
 
