@@ -110,7 +110,8 @@ ks_status ks_ctx_set_wait_limit(ks_ctx *ctx, int64_t ns);
  * increasing column order, with the diagonals at least 3/4 full, also keeps
  * a diagonal copy (values diagonal-major, one presence mask byte per row),
  * which the SpMV reads instead of the CSR arrays: no column indices at all,
- * coalesced reads of x. Results are identical. This flag keeps CSR only. */
+ * coalesced reads of x. Results are identical. This flag keeps CSR only (nor is
+ * there the sliced copy that CG on other matrices of that size reads). */
 #define KS_MAT_NO_DIAG 16u
 
 /* Upload a host CSR matrix (collection::CudaCopy_Part1,

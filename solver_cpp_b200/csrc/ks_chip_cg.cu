@@ -70,6 +70,11 @@ cudaError_t tile_launch(ks_ctx *ctx, const CsrDev &A, const ChipArgs &a, const C
   return coop_launch(ctx, "k_cg_tile", k_cg_tile, sh, probe, fits, cls, kChipThreads, a, D);
 }
 
+bool csr_window_fits(const ks_ctx *ctx, long long n, int lo, int hi) {
+  CsrShape s;
+  return csr_shape(ctx, n, lo, hi, &s);
+}
+
 cudaError_t csr_launch(ks_ctx *ctx, const CsrCgArgs &a, const CsrShape &sh, bool probe, bool *fits, int cls) {
   auto run = [&](auto kern) { return coop_launch(ctx, "k_cg_csr", kern, sh, probe, fits, cls, sh.threads, a); };
   if (sh.threads == 1024) return run(k_cg_csr<1024, 4>);  // more than 2,048 rows per CTA

@@ -1003,11 +1003,11 @@ struct CsrShape : ChipShape {
   int wl = 0, wu = 0;
 };
 
-// The CTAs of chip_ctas. False
-// where the matrix has no slices or its window does not fit.
-inline bool csr_shape(const ks_ctx *ctx, const CsrDev &A, long long n, CsrShape *s) {
+// The CTAs of chip_ctas; lo, hi: the matrix's largest offsets. False where the
+// window does not fit.
+inline bool csr_shape(const ks_ctx *ctx, long long n, int lo, int hi, CsrShape *s) {
   const long long sms = std::min(ctx->num_sms, (int)kChipMaxGrid);
-  if (!A.sell_val || n < 1 || n != A.n || n > sms * kCsrRows * 1024) return false;
+  if (n < 1 || n > sms * kCsrRows * 1024) return false;
   int optin = 0;
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -1020,8 +1020,8 @@ inline bool csr_shape(const ks_ctx *ctx, const CsrDev &A, long long n, CsrShape 
   s->rj = 1;
   s->threads = s->rpc <= kCsrRows * 512 ? 512 : 1024;
   while (s->rj * s->threads < s->rpc) s->rj *= 2;
-  s->wl = A.sell_lo;
-  s->wu = A.sell_hi;
+  s->wl = lo;
+  s->wu = hi;
   s->smem = sizeof(double) * ((size_t)s->rpc + s->wl + s->wu);
   return s->rj <= kCsrRows && s->smem + 2048 <= (size_t)optin;
 }

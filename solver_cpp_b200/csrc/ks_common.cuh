@@ -85,7 +85,8 @@ struct CsrDev {
   // sell_off (col - row). Kept for matrices without a diagonal copy, up to 4,096
   // rows per SM, whose offsets fit in 16 bits and whose slices hold no more than
   // twice the nonzeros; sell_lo, sell_hi: the largest offsets below and above
-  // the row. Null otherwise.
+  // the row. Only where the window those span fits in shared memory, and not with
+  // KS_MAT_NO_DIAG. Null otherwise.
   int *sell_ptr = nullptr;
   double *sell_val = nullptr;
   short *sell_off = nullptr;
@@ -401,6 +402,10 @@ ks_status cuda_fail(ks_ctx *ctx, cudaError_t e, const char *what);
 int red_grid(const ks_ctx *ctx);  // CTAs of the vector kernels
 // Reads and clears the context's timeout flag (synchronises the stream).
 ks_status check_device_error(ks_ctx *ctx);
+
+// Whether p of a CTA's rows and of those within the offsets lo below and hi above
+// fits in shared memory (k_cg_csr; ks_chip_cg.cu).
+bool csr_window_fits(const ks_ctx *ctx, long long n, int lo, int hi);
 
 // Workspace pool (device buffers reused across solves).
 ks_status pool_get(ks_ctx *ctx, size_t bytes, void **out);

@@ -209,10 +209,11 @@ __global__ void k_to_bf16(const double *__restrict__ a, __nv_bfloat16 *__restric
 // Checks every column index (cmin <= col < cmax) and stores col - row as
 // int16 where it fits: flags |= 1 for a column out of range, |= 2 for an
 // offset outside [-32768, 32767] (col16 is then discarded by the caller).
+// flags[1], flags[2]: the largest of the other offsets below and above a row.
 // Rows of a split solve store col - r0, so col - row is the global offset.
 __global__ void k_col16(const int *__restrict__ ptr, const int *__restrict__ col, int n, long long cmin,
                         long long cmax, short *__restrict__ col16, int *flags) {
-  int bad = 0;
+  int bad = 0, lo = 0, hi = 0;
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n;
        r += (long long)gridDim.x * blockDim.x) {
     const int j1 = ptr[r + 1];
@@ -223,13 +224,24 @@ __global__ void k_col16(const int *__restrict__ ptr, const int *__restrict__ col
         continue;
       }
       const int d = c - (int)r;
-      if (d < -32768 || d > 32767)
+      if (d < -32768 || d > 32767) {
         bad |= 2;
-      else if (col16)
-        col16[j] = (short)d;
+        continue;
+      }
+      lo = max(lo, -d);
+      hi = max(hi, d);
+      if (col16) col16[j] = (short)d;
     }
   }
   if (bad) atomicOr(flags, bad);
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(flags + 1, lo);
+    atomicMax(flags + 2, hi);
+  }
 }
 
 // Diagonal copy (CsrDev::dia_*), pass 1: the distinct offsets col - row of
@@ -556,11 +568,10 @@ static ks_status build_diagonals(ks_ctx *ctx, CsrDev &A, unsigned flags, long lo
 }
 
 // The slices of k_cg_csr (CsrDev::sell_*): one warp per slice of 32 rows, lane =
-// row. range: the largest offset below and above a row.
+// row.
 __global__ void k_sell_fill(const int *__restrict__ ptr, const short *__restrict__ col16, const double *__restrict__ val,
-                            int n, const int *__restrict__ slice, double *__restrict__ sval, short *__restrict__ soff,
-                            int *range) {
-  int lo = 0, hi = 0;
+                            int n, const int *__restrict__ slice, double *__restrict__ sval,
+                            short *__restrict__ soff) {
   const int lane = threadIdx.x & 31, warps = gridDim.x * blockDim.x / 32;
   for (int s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < (n + 31) / 32; s += warps) {
     const int i = 32 * s + lane, j0 = i < n ? ptr[i] : 0, len = i < n ? ptr[i + 1] - j0 : 0;
@@ -570,22 +581,15 @@ __global__ void k_sell_fill(const int *__restrict__ ptr, const short *__restrict
       const int o = k < len ? col16[j0 + k] : 0;
       sval[e] = k < len ? val[j0 + k] : 0.0;
       soff[e] = (short)o;
-      lo = max(lo, -o);
-      hi = max(hi, o);
     }
-  }
-  for (int d = 16; d > 0; d >>= 1) {
-    lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
-  }
-  if (lane == 0) {
-    atomicMax(range, lo);
-    atomicMax(range + 1, hi);
   }
 }
 
-// An optimisation: where the device cannot hold the copy there is none.
-static ks_status build_slices(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr) {
+// lo, hi: the largest offsets below and above a row. None where k_cg_csr's window
+// does not fit. An optimisation: where the device cannot hold the copy there is
+// none either.
+static ks_status build_slices(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr, int lo, int hi) {
+  if (!csr_window_fits(ctx, A.n, lo, hi)) return KS_OK;
   const int ns = (A.n + 31) / 32;
   std::vector<int> sp((size_t)ns + 1, 0);
   for (int s = 0; s < ns; s++) {
@@ -596,31 +600,21 @@ static ks_status build_slices(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr) {
     sp[s + 1] = (int)next;
   }
   const size_t total = 32 * (size_t)sp[ns];
-  int *range = nullptr;
-  int h[2] = {0, 0};
   cudaError_t e = cudaMalloc(&A.sell_ptr, sizeof(int) * sp.size());
   if (e == cudaSuccess) e = cudaMalloc(&A.sell_off, sizeof(short) * std::max<size_t>(total, 1));
   if (e == cudaSuccess) e = cudaMalloc(&A.sell_val, sizeof(double) * std::max<size_t>(total, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&range, sizeof(h));
   if (e == cudaErrorMemoryAllocation) {
     (void)cudaGetLastError();
   } else {
     if (e == cudaSuccess) e = cudaMemcpyAsync(A.sell_ptr, sp.data(), sizeof(int) * sp.size(), cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(range, 0, sizeof(h), ctx->stream);
     if (e == cudaSuccess) {
-      k_sell_fill<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(A.ptr, A.col16, A.val, A.n, A.sell_ptr, A.sell_val, A.sell_off,
-                                                            range);
+      k_sell_fill<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(A.ptr, A.col16, A.val, A.n, A.sell_ptr, A.sell_val, A.sell_off);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, range, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // sp goes out of scope, too
-    if (e != cudaSuccess) {
-      cudaFree(range);
-      return cuda_fail(ctx, e, "matrix slices");
-    }
-    A.sell_lo = h[0];
-    A.sell_hi = h[1];
-    cudaFree(range);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // sp goes out of scope
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "matrix slices");
+    A.sell_lo = lo;
+    A.sell_hi = hi;
     return KS_OK;
   }
   cudaFree(A.sell_ptr);
@@ -677,24 +671,25 @@ static ks_status finish_csr(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr, uns
                                ctx->stream));
   const long long tot = A.nnz + kPad;
   const int g = ctx->num_sms * 8;
+  int h_flags[3] = {0, 0, 0};  // k_col16's flags and offsets
   {
     if (!(flags & KS_MAT_INDEX32)) {
       KS_CUDA(ctx, cudaMalloc(&A.col16, sizeof(short) * (size_t)tot));
       KS_CUDA(ctx, cudaMemsetAsync(A.col16 + A.nnz, 0, sizeof(short) * kPad, ctx->stream));
     }
-    int *d_flags = nullptr, h_flags = 0;
-    KS_CUDA(ctx, cudaMalloc(&d_flags, sizeof(int)));
-    cudaError_t e = cudaMemsetAsync(d_flags, 0, sizeof(int), ctx->stream);
+    int *d_flags = nullptr;
+    KS_CUDA(ctx, cudaMalloc(&d_flags, sizeof(h_flags)));
+    cudaError_t e = cudaMemsetAsync(d_flags, 0, sizeof(h_flags), ctx->stream);
     if (e == cudaSuccess) {
       k_col16<<<g, 256, 0, ctx->stream>>>(A.ptr, A.col, A.n, cmin, cmax, A.col16, d_flags);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_flags, d_flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_flags, d_flags, sizeof(h_flags), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_flags);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "column index check");
-    if (h_flags & 1) return set_error(ctx, KS_BAD_INPUT, "column index out of range");
-    if (h_flags & 2) {
+    if (h_flags[0] & 1) return set_error(ctx, KS_BAD_INPUT, "column index out of range");
+    if (h_flags[0] & 2) {
       cudaFree(A.col16);
       A.col16 = nullptr;
     }
@@ -709,8 +704,8 @@ static ks_status finish_csr(ks_ctx *ctx, CsrDev &A, const int32_t *host_ptr, uns
   }
   KS_CUDA(ctx, cudaGetLastError());
   if (!(flags & KS_MAT_NO_DIAG)) KS_TRY(build_diagonals(ctx, A, flags, cmin, cmax));
-  if (!A.dia_nd && A.col16 && cmin == 0 && cmax == A.n && A.n > kSliceMinRows && A.n <= 4096LL * ctx->num_sms)
-    KS_TRY(build_slices(ctx, A, host_ptr));
+  if (!(flags & KS_MAT_NO_DIAG) && !A.dia_nd && A.col16 && cmin == 0 && cmax == A.n && A.n > kSliceMinRows && A.n <= 4096LL * ctx->num_sms)
+    KS_TRY(build_slices(ctx, A, host_ptr, h_flags[1], h_flags[2]));
   // rb and rbi are host vectors going out of scope: the copies must complete first.
   KS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return KS_OK;

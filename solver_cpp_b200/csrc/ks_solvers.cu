@@ -853,7 +853,7 @@ inline bool run_cg_csr(const Env<double> &E, const double *b, double *x, double 
   ks_ctx *ctx = E.ctx;
   const CsrDev &A = *E.A;
   CsrShape sh;
-  if (!csr_shape(ctx, A, E.n, &sh)) return false;
+  if (!A.sell_val || A.n != E.n || !csr_shape(ctx, E.n, A.sell_lo, A.sell_hi, &sh)) return false;
   CsrCgArgs a{};
   static_cast<IrArgs &>(a) = IrArgs{b, x, R, E.st, nullptr, ctx->partials, (IrSync *)ctx->ir_sync, ctx->d_err, ctx->wait_ns,
                                     (int)E.n, sh.rpc, sh.rj, 1, 0};
