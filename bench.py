@@ -179,22 +179,25 @@ def barrier(world):
         dist.barrier()
 
 
-def spmv_bytes(n, nnz, values, index_bytes=4, diagonals=0, symmetric=0):
+def spmv_bytes(n, nnz, values, index_bytes=4, diagonals=0, symmetric=0, constant=0):
     """Algorithmic bytes of one SpMV. CSR: values + column indices (int32, or
     the int16 row offsets the library stores when they fit) + int32 row
     offsets + x read once + y written once. Diagonal copy (`diagonals` > 0):
     the stored diagonals' values (zeros where a row has no entry; a symmetric
-    matrix stores its main and upper diagonals only) + one mask byte per row
-    for FP64 + x read once + y written once."""
+    matrix stores its main and upper diagonals only; `constant` ones of one value
+    each are the FP64 kernel's parameters) + one mask byte per row for FP64 + x
+    read once + y written once."""
     vb = {"fp64": 8, "fp32": 4, "bf16": 2}[values]
     xb = 8 if values == "fp64" else 4
     if diagonals:
         stored = diagonals // 2 + 1 if symmetric else diagonals
+        if constant and values == "fp64":
+            stored = 0
         return stored * n * vb + (n if values == "fp64" else 0) + xb * n + xb * n
     return nnz * (vb + index_bytes) + 4 * (n + 1) + xb * n + xb * n
 
 
-def onchip_inner_bytes(n, values, diagonals, symmetric, info, iters, sms=148):
+def onchip_inner_bytes(n, values, diagonals, symmetric, info, iters, sms=148, constant=0):
     """Algorithmic bytes of one launch of the on-chip CG kernel (vectors on
     chip, the matrix read every iteration): per iteration the stored
     diagonals' values (and one mask byte per row with FP64 values), p
@@ -202,10 +205,13 @@ def onchip_inner_bytes(n, values, diagonals, symmetric, info, iters, sms=148):
     ceil(n / sms) rows, and reads the rows an offset reaches beyond its own,
     at each end); once: the right-hand side read and x written. Vectors are
     FP32 for the inner solve of a VP method (fp32 / bf16 values) and FP64 for
-    a whole FP64 solve (fp64 values)."""
+    a whole FP64 solve (fp64 values), which reads no values of `constant`
+    diagonals."""
     vb = {"fp64": 8, "fp32": 4, "bf16": 2}[values]
     xb = 8 if values == "fp64" else 4
     stored = diagonals // 2 + 1 if symmetric else diagonals
+    if constant and values == "fp64":
+        stored = 0
     rpc = -(-n // sms)
     offs = info.get("offsets") or []
     halo = sum(min(abs(int(o)), rpc) for o in offs if o) * sms
@@ -213,18 +219,36 @@ def onchip_inner_bytes(n, values, diagonals, symmetric, info, iters, sms=148):
     return iters * (stored * n * vb + mask + xb * n + xb * halo) + 2 * xb * n
 
 
-def onchip_whole_bytes(method, n, diagonals, symmetric, info, iters, sms=148):
+def onchip_whole_bytes(method, n, diagonals, symmetric, info, iters, sms=148, constant=0):
     """Algorithmic bytes of a whole FP64 solve as one on-chip launch that reads
-    the matrix in every iteration (k_cg_chip and k_cg_tile hold it on chip and
-    move less): CG as onchip_inner_bytes; CR also updates x in place in global memory (read and
-    written every iteration, 16 n); BiCG runs two SpMVs per iteration (A and
-    A^T: both diagonal copies, masks, published vectors and halos)."""
-    one = onchip_inner_bytes(n, "fp64", diagonals, symmetric, info, iters, sms)
+    the matrix in every iteration: CG as onchip_inner_bytes; CR also updates x in
+    place in global memory (read and written every iteration, 16 n); BiCG runs two
+    SpMVs per iteration (A and A^T: both diagonal copies, masks, published vectors
+    and halos)."""
+    one = onchip_inner_bytes(n, "fp64", diagonals, symmetric, info, iters, sms, constant)
     if method == "CR":
         return one + iters * 16 * n
     if method == "BICG":
         return 2 * one - 16 * n
     return one
+
+
+def held_bytes(kernel, n, values, diagonals, symmetric):
+    """Algorithmic bytes of one launch of a CG kernel that holds the matrix on chip:
+    k_cg_chip reads its stored diagonals once, k_cg_tile has them as parameters;
+    the right-hand side read and x written. None for the other kernels."""
+    if kernel not in ("k_cg_chip", "k_cg_tile"):
+        return None
+    vb = {"fp64": 8, "fp32": 4, "bf16": 2}[values]
+    stored = diagonals // 2 + 1 if symmetric else diagonals
+    return n * ((stored * vb if kernel == "k_cg_chip" else 0) + 2 * (8 if values == "fp64" else 4))
+
+
+def constant_diagonals(A):
+    """Whether each diagonal of A (offset col - row) holds one value, bit for bit."""
+    off = A.col.astype(np.int64) - np.repeat(np.arange(A.n, dtype=np.int64), np.diff(A.ptr))
+    bits = np.ascontiguousarray(A.val).view(np.int64)
+    return all(np.unique(bits[off == o]).size == 1 for o in np.unique(off))
 
 
 def layout_key(info):
@@ -338,6 +362,7 @@ def run_ours(args, world, rank, local):
     if nd:  # the diagonals' offsets col - row, from the host matrix
         rows = np.repeat(np.arange(A.n, dtype=np.int64), np.diff(A.ptr))
         minfo["offsets"] = [int(o) for o in np.unique(A.col.astype(np.int64) - rows)]
+    cst = int(bool(nd) and constant_diagonals(A))
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=f"cuda:{local}")  # larger than the 126 MB L2
 
     def time_launches(fn, reps=50, cold=False, clean=True):
@@ -377,7 +402,7 @@ def run_ours(args, world, rank, local):
         fn = lambda: ks.spmv(M, xs, ys, values=vcode)  # noqa: E731
         warm, cold = time_launches(fn), time_launches(fn, reps=20, cold=True)
         dirty = time_launches(fn, reps=20, cold=True, clean=False)
-        alg = spmv_bytes(nl, nnzl, vals, ib, nd, sym)
+        alg = spmv_bytes(nl, nnzl, vals, ib, nd, sym, cst)
         spmv[vals] = {"alg_bytes": alg, "launch_ms": round(warm, 5), "launch_ms_cold": round(cold, 5),
                       "gbs": round(alg / (warm / 1e3) / 1e9, 1), "frac": round(alg / (warm / 1e3) / 1e9 / peak, 4),
                       "frac_cold": round(alg / (cold / 1e3) / 1e9 / peak, 4),
@@ -388,6 +413,7 @@ def run_ours(args, world, rank, local):
 
     # In the solve: one solve with per-class device times
     prof = ks.solve(ctx, M, W["outer"], B, inner=W["inner"], x=X, profile=1, **W["params"]).report
+    kname = ctx.solve_kernel()  # the one that ran the solve (its inner solves) in one launch
     vals = W["spmv_values"]
     inner_calls = res.inner_calls
     onchip_inner = W["inner"] != "NONE" and prof["n_mv_low"] > 0 and prof["n_mv_low"] <= inner_calls + 1
@@ -397,12 +423,15 @@ def run_ours(args, world, rank, local):
         # the dominant kernel: one inner solve of `l` CG iterations on chip
         iters = int(W["params"]["l"])
         per_launch_ms = prof["t_mv_low"] / max(1, prof["n_mv_low"]) * 1e3
-        alg = onchip_inner_bytes(nl, vals, nd, sym, minfo, iters)
+        held = held_bytes(kname, nl, vals, nd, sym)
+        alg = held if held is not None else onchip_inner_bytes(nl, vals, nd, sym, minfo, iters)
         if os.path.exists(tf):
             traffic = json.load(open(tf)).get(f"{args.workload}:onchip_inner:{vals}")
-        roofline = {"bound": "hbm", "achieved": round(alg / (per_launch_ms / 1e3) / 1e9, 1), "peak": peak,
-                    "unit": "GB/s", "frac": round(alg / (per_launch_ms / 1e3) / 1e9 / peak, 4), "traffic": traffic,
-                    "kernel": f"k_cg_onchip (one inner CG solve of {iters} iterations, vectors on chip, "
+        roofline = {"bound": "hbm" if held is None else "on-chip latency",
+                    "achieved": round(alg / (per_launch_ms / 1e3) / 1e9, 1), "peak": peak,
+                    "unit": "GB/s", "frac": round(alg / (per_launch_ms / 1e3) / 1e9 / peak, 4),
+                    "traffic": traffic if held is None else None,
+                    "kernel": f"{kname} (one inner CG solve of {iters} iterations, vectors on chip, "
                               f"{vals} values)",
                     "alg_bytes_per_launch": alg, "launch_ms": round(per_launch_ms, 5),
                     "us_per_inner_iteration": round(per_launch_ms * 1e3 / iters, 3),
@@ -415,19 +444,14 @@ def run_ours(args, world, rank, local):
         # the whole FP64 solve as one on-chip launch (profiled as one SpMV-class launch)
         iters = max(1, int(res.loop) - 1)  # the stopping test at the top of iteration `loop`
         launch_ms = prof["t_mv"] * 1e3
-        alg = onchip_whole_bytes(W["outer"], nl, nd, sym, minfo, iters)
-        # CG that holds the matrix on chip as well (k_cg_chip), or constant diagonals
-        # as its parameters (k_cg_tile): the diagonals, b and x once
-        held = W["outer"] == "CG" and (nl <= 148 * 4096 or W["problem"] == "poisson3d")
-        if held:
-            alg = nl * (8 * (nd // 2 + 1 if sym else nd) + 1 + 16)
-        kname = {"CG": "on-chip CG kernel", "CR": "k_cr_onchip", "BICG": "k_bicg_onchip"}[W["outer"]]
+        held = held_bytes(kname, nl, "fp64", nd, sym)
+        alg = held if held is not None else onchip_whole_bytes(W["outer"], nl, nd, sym, minfo, iters, constant=cst)
         if os.path.exists(tf):
             traffic = json.load(open(tf)).get(f"{args.workload}:onchip_whole:fp64")
-        roofline = {"bound": "on-chip latency" if held else "hbm",
+        roofline = {"bound": "hbm" if held is None else "on-chip latency",
                     "achieved": round(alg / (launch_ms / 1e3) / 1e9, 1), "peak": peak,
                     "unit": "GB/s", "frac": round(alg / (launch_ms / 1e3) / 1e9 / peak, 4),
-                    "traffic": None if held else traffic,
+                    "traffic": traffic if held is None else None,
                     "kernel": f"{kname} (the whole {W['outer']} solve, {iters} iterations, vectors on chip, fp64)",
                     "alg_bytes_per_launch": alg, "launch_ms": round(launch_ms, 5),
                     "us_per_iteration": round(launch_ms * 1e3 / max(1, iters), 3),
