@@ -18,9 +18,10 @@
 // and, behind a flag per CTA, fetched by all warps but the first while the (r, r)
 // sum travels. What bounds it: the L2 reads of the matrix (35 MB of values and
 // offsets here), the bank conflicts of the gathers, and the two grid sums. Measured,
-// us per iteration, one kernel per step (9,000 rows: one cluster) / k_cg_csr: 9,000
-// rows of 14 entries 11.5 / 6.1, 100K of 20 39 / 11.0, 250K of 14 41 / 13.9, 600K of
-// 7 44 / 20.4.
+// us per iteration, one kernel per step (up to 32K rows: one cluster) / k_cg_csr:
+// 9,000 rows of 14 entries 11.5 / 6.1, 20K 28 / 8.0, 40K 18 / 10.0, 60K 20 / 12.2, 100K
+// of 20 39 / 11.0, 250K of 14 41 / 13.9, of 50 107 / 54, 600K of 7 44 / 20.4, of 27
+// 162 / 50 (the matrices of 250K x 50 and 600K x 27 do not fit in L2).
 #pragma once
 
 #include "ks_chip_cg.cuh"

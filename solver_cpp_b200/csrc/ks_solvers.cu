@@ -809,9 +809,10 @@ constexpr long long kChipMinRows = 8192;
 // Larger systems whose matrix fits on chip across the GPU as well as their
 // vectors (up to about 4,096 rows per SM in FP64, one GPU, a diagonal copy;
 // ks_params.cluster_solve 0), or constant-coefficient 7-point stencils on a box
-// whose vectors do (up to about 16,000 rows per SM): the whole solve as one cooperative kernel
-// (k_cg_chip, ks_chip_cg.cuh; k_cg_tile, ks_tile_cg.cuh). Returns false, having
-// launched nothing, when the system does not qualify.
+// whose vectors do and that a tile fits (tile_shape; up to about 16,000 rows per SM):
+// the whole solve as one cooperative kernel (k_cg_chip, ks_chip_cg.cuh; k_cg_tile,
+// ks_tile_cg.cuh). Returns false, having launched nothing, when the system does not
+// qualify.
 inline bool run_cg_chip(const Env<double> &E, const double *b, double *x, double *R, ks_status *s) {
   if (E.sp.cluster_solve || !E.outer || E.comm || E.mvals != KS_FP64 || !E.A->dia_nd || !E.A->dia_val) return false;
   if (reinterpret_cast<uintptr_t>(R) % 16) return false;  // R takes the first two workspace slots

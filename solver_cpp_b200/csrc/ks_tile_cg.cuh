@@ -1,7 +1,11 @@
 // CG on tiles of a box, the vectors on chip (sm_100a): FP64 CG of 7-point
 // stencils on a box whose diagonals each hold one value, every entry of the box
-// present (CsrDev::dia_box 2, dia_cst: Poisson), above the size whose values fit
-// on chip (k_cg_chip, about 600K rows) up to about 2.4M rows.
+// present (CsrDev::dia_box 2, dia_cst: Poisson) and every value finite, above the
+// size whose values fit on chip (k_cg_chip, about 600K rows), where a tile fits
+// (tile_shape: 1,440 rows of a plane, 1,920 of a face in y, 32 rows per thread and p
+// in shared memory at most). That is cubes up to 128^3 and about three of four boxes
+// of random edges (20 to 260) between 606K and 2.4M rows; the others, 130 x 127 x
+// 129 or lines of 1,200 rows, take k_cg_onchip.
 //
 // A CTA owns a tile of by x bz whole lines of the box (k_cg_chip's tiles):
 // p of its rows and of the lines around them in shared memory, each line
@@ -12,20 +16,21 @@
 // constant and p[z - 1], p[z] stay in registers. The rows of a block are computed
 // without branches, those past the tile's last plane on its place and then
 // dropped: with a branch per row the FP64 chains of a product run one after
-// another (128^3: 13,400 clocks per product, now 10,000). (Rows t + 512 j
-// with their places computed one by one: 120 of 156 instructions per row and
-// iteration were index arithmetic.)
+// another (128^3: 13,400 clocks per product, without 10,000). An iteration executes
+// 123 instructions per row. (Rows t + 512 j with their places computed one by one:
+// 156, of which 120 were index arithmetic.)
 // k_cg_onchip's runs of consecutive rows read two planes of p through L2 per
-// product (160^3: 51,200 rows for a CTA's 27,680); a tile reads the 2 (by + bz)
-// lines of its faces (9,000 rows for 28,800) once, into shared memory.
+// product (128^3: 32,768 rows for a CTA's 14,176); a tile reads the 2 (by + bz)
+// lines of its faces (8 x 15 lines: 5,888 rows for 15,360) once, into shared memory.
 //
 // r crosses between CTAs in the shadow of the (r, r) sum: the rows in another
 // CTA's halo are stored to R, then (behind the barrier of the sum's post) a
 // thread of warp 1 releases the CTA's flag, acquires the neighbours' and lets
 // warps 1 .. 15 load the halo; warp 0 meanwhile waits for the sum. Tags with
-// every value, as k_cg_chip has, cost 50-60 clocks per warp access (128^3 FP64,
-// 5,632 halo rows per CTA: 22.8 us per iteration with them), and flags acquired
-// by all 16 warps more still: the polls of 148 CTAs delay the stores.
+// every value, as k_cg_chip has, cost 50-60 clocks per warp access (an earlier form
+// of this kernel at 128^3, tiles of 10 x 12 lines: 22.8 us per iteration with tags,
+// 20.9 with flags), and flags acquired by all 16 warps more still: the polls of 148
+// CTAs delay the stores.
 //
 // The matrix is the kernel's parameters: an iteration moves nothing but the
 // halo. (The same kernel with the values of other matrices read from L2 in every
@@ -35,10 +40,11 @@
 // an absent entry's term is a zero added to a sum that starts at +0.
 //
 // What bounds an iteration: shared memory (5 reads of 8 bytes per row in A, 1 and
-// 2 in the updates: 128^3, 15,360 rows per CTA, 7,700 of 36,000 clocks), the FP64
-// pipe and its latency, and the two grid sums (3,200 each). Measured, us per
-// iteration, k_cg_onchip / k_cg_tile: 100^3 20.9 / 11.1, 128^3 35.7 (26.3 with the
-// diagonals as parameters) / 17.0.
+// 2 in the updates: 128^3, 15,360 rows per CTA, 7,700 of 30,700 clocks), the FP64
+// pipe (19 % busy) and its latency, and the two grid sums (3,200 each). Measured, us
+// per iteration, k_cg_onchip / k_cg_tile: 100^3 20.9 / 10.6, 128^3 35.7 (26.3 with
+// the diagonals as parameters) / 15.6. Where a block's loads in p = beta p + r were not
+// issued before its stores: 128^3 16.8.
 #pragma once
 
 #include "ks_chip_cg.cuh"
