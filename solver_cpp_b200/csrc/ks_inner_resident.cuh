@@ -600,11 +600,11 @@ __device__ __forceinline__ void ir_p4(const VT *sp, const VT *P, int r0, int nr,
   }
 }
 
-// kC: every diagonal's entries are one value (DiaT::cst): the values come from
+// kC: every diagonal's entries are one value (DiaC): the values come from
 // the kernel's parameters and nothing is read. A template parameter of the
 // kernels: chosen at run time inside them, the two ways spill registers.
-template <bool kC, class MT>
-__device__ __forceinline__ bool ir_const(const DiaT<MT> &D, int d, IrVals<MT> &v) {
+template <bool kC, class Dia, class MT>
+__device__ __forceinline__ bool ir_const(const Dia &D, int d, IrVals<MT> &v) {
   if constexpr (kC) {
 #pragma unroll
     for (int e = 0; e < kIrQ; e++) v.v[e] = D.cv[d];
@@ -620,7 +620,7 @@ __device__ __forceinline__ bool ir_const(const DiaT<MT> &D, int d, IrVals<MT> &v
 // warp). Every diagonal's value is loaded (zeros where a row has none); FP64
 // adds only the terms the row's mask names, FP32 adds every one.
 template <class VT, class MT, int NDG, bool kC>
-__device__ __forceinline__ void ir_quad_mv(const DiaT<MT> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
+__device__ __forceinline__ void ir_quad_mv(const DiaOf<MT, kC> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
                                            int nd, VT (&q)[kIrQ]) {
   constexpr int KD = NDG > 0 ? NDG : kMaxDiag;
   constexpr int B = sizeof(MT) == 2 ? KD : (sizeof(MT) == 4 ? 4 : 2);  // diagonals per batch
@@ -716,7 +716,7 @@ __device__ __forceinline__ VT ir_val(const IrVals<MT> &a, int e) {
 // that starts at +0, which leaves it unchanged, so the terms and their order
 // are ir_quad_mv's and so are the results.
 template <class VT, class MT, int NDG, bool kC>
-__device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
+__device__ __forceinline__ void ir_quad_mv_st(const DiaOf<MT, kC> &D, const VT *P, const VT *sp, int r0, int nr, int li0,
                                               const VT (&pv)[kIrQ], VT (&q)[kIrQ]) {
   static_assert(NDG == 5 || NDG == 7, "stencil path: 5 or 7 diagonals");
   constexpr int H = NDG / 2;  // the main diagonal
@@ -731,9 +731,10 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
   IrVals<MT> vm1, v1;
   if (!ir_const<kC>(D, H + 1, v1)) ir_vals4<MT>(D.vb[H + 1] + i0, v1);
   MT m1s = (MT)0;
-  if (ir_const<kC>(D, H - 1, vm1))
+  if constexpr (kC) {
+    ir_const<kC>(D, H - 1, vm1);
     m1s = D.cv[H - 1];
-  else if (sym)
+  } else if (sym)
     m1s = ir_ld<MT>(D.vb[H + 1] + (i0 - 1));
   else
     ir_vals4<MT>(D.vb[H - 1] + i0, vm1);
@@ -801,7 +802,7 @@ __device__ __forceinline__ void ir_quad_mv_st(const DiaT<MT> &D, const VT *P, co
 // The solve (see the top of this file). Returns the stopping code, or -1
 // when a wait ran out; *xw: x was written (one update at least).
 template <class VT, class MT, int NDG, bool kC>
-__device__ __forceinline__ int ir_body(const DiaT<MT> &D, const IrArgs &a, VT *sp, VT *sx, uint32_t tm,
+__device__ __forceinline__ int ir_body(const DiaOf<MT, kC> &D, const IrArgs &a, VT *sp, VT *sx, uint32_t tm,
                                        long long *Lout, double *alpha_out, double *beta_out, double *rr_out,
                                        bool *xw) {
   using TW = IrWords<VT>;
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ int ir_body(const DiaT<MT> &D, const IrArgs &a, VT *s
 }
 
 template <class VT, class MT, int NDG, bool kC = false>
-__global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaT<MT> D, IrArgs a) {
+__global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaOf<MT, kC> D, IrArgs a) {
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
   __shared__ uint32_t s_tmem;
   VT *sp = reinterpret_cast<VT *>(ir_smem_raw);  // p of the CTA's rows
@@ -1098,7 +1099,7 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_cg_onchip(DiaT<MT> D, IrArgs 
 constexpr int kIbVecs = 6;
 
 template <int NDG, bool kC>
-__global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaT<double> DA, DiaT<double> DT, IrArgs a) {
+__global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaOf<double, kC> DA, DiaOf<double, kC> DT, IrArgs a) {
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
   double *sx = reinterpret_cast<double *>(ir_smem_raw);
   double *sr = sx + a.rpc, *srs = sr + a.rpc, *sp = srs + a.rpc, *sps = sp + a.rpc, *sq = sps + a.rpc;
@@ -1141,7 +1142,7 @@ __global__ void __launch_bounds__(kIrThreads, 1) k_bicg_onchip(DiaT<double> DA, 
         if (li0 + e < nr) __stcg(G + r0 + li0 + e, o[e]);
     }
   };
-  auto mv = [&](const DiaT<double> &D, const double *G, const double *sv, const double (&own)[kIrQ],
+  auto mv = [&](const DiaOf<double, kC> &D, const double *G, const double *sv, const double (&own)[kIrQ],
                 double (&y)[kIrQ]) {
     bool done = false;
     if constexpr (NDG == 5 || NDG == 7) {
@@ -1333,7 +1334,7 @@ inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, co
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, kMv);  // a profiled solve counts the whole solve as one SpMV-class launch
-  return cudaLaunchKernelEx(&cfg, fn, dview<double>(A), dview<double>(T), a);
+  return cudaLaunchKernelEx(&cfg, fn, dview_of<kC, double>(A), dview_of<kC, double>(T), a);
 }
 
 
@@ -1353,7 +1354,7 @@ inline cudaError_t ib_launch_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, co
 // Three grid reductions and no publication wait per iteration; element
 // operations are the engine's, only the dot sums' order differs.
 template <int NDG, bool kC>
-__global__ void __launch_bounds__(kIrThreads, 1) k_cr_onchip(DiaT<double> D, IrArgs a) {
+__global__ void __launch_bounds__(kIrThreads, 1) k_cr_onchip(DiaOf<double, kC> D, IrArgs a) {
   using TW = IrWords<double>;
   extern __shared__ __align__(16) unsigned char ir_smem_raw[];
   __shared__ uint32_t s_tmem;
@@ -1723,7 +1724,7 @@ inline cudaError_t ir_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, co
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, cls);
-  return cudaLaunchKernelEx(&cfg, fn, dview<MT>(A), a);
+  return cudaLaunchKernelEx(&cfg, fn, dview_of<kC, MT>(A), a);
 }
 
 template <class VT, class MT, int NDG>
@@ -1768,7 +1769,7 @@ inline cudaError_t icr_launch_n(ks_ctx *ctx, const CsrDev &A, const IrArgs &a, c
   ctx->launches++;
   ctx->ir_used = true;  // its matrix lines are evict_last in L2 (ir_l2_release)
   ProfLaunch pl(ctx, kMv);  // a profiled solve counts the whole solve as one SpMV-class launch
-  return cudaLaunchKernelEx(&cfg, fn, dview<double>(A), a);
+  return cudaLaunchKernelEx(&cfg, fn, dview_of<kC, double>(A), a);
 }
 
 }  // namespace ks

@@ -386,8 +386,16 @@ inline DiaT<MT> dview(const CsrDev &A) {
   d.cmax = A.dia_cmax;
   for (int k = 0; k < kMaxDiag; k++) d.off[k] = A.dia_off[k];
   d.quad = 0;
-  d.cst = std::is_same<MT, double>::value ? A.dia_cst : 0;
-  for (int k = 0; k < kMaxDiag; k++) d.cv[k] = (MT)(d.cst ? A.dia_cv[k] : 0.0);
+  return d;
+}
+
+// The view a kernel with or without kC takes (of a matrix with dia_cst for kC).
+template <bool kC, class MT>
+inline DiaOf<MT, kC> dview_of(const CsrDev &A) {
+  DiaOf<MT, kC> d;
+  static_cast<DiaT<MT> &>(d) = dview<MT>(A);
+  if constexpr (kC)
+    for (int k = 0; k < kMaxDiag; k++) d.cv[k] = (MT)A.dia_cv[k];
   return d;
 }
 
@@ -438,8 +446,8 @@ inline void launch_spmv_dn(ks_ctx *ctx, const CsrDev &A, const GX &g0, const GX 
     dv.quad = dia_quad_ok(A, g0.x, epi.y) ? 1 : 0;
   if constexpr (std::is_same<MT, double>::value) {
     if (A.dia_cst) {  // on the same grid: sums in its epilogue add their terms in the same order
-      launch_k(ctx, spmv_dia_kernel<NV, NDG, MT, GX, Epi, true>, dim3(grid), dim3(kThreads), 0, dv, g0, g1, epi, stop,
-               red_of(ctx, slot));
+      launch_k(ctx, spmv_dia_kernel<NV, NDG, MT, GX, Epi, true>, dim3(grid), dim3(kThreads), 0,
+               dview_of<true, MT>(A), g0, g1, epi, stop, red_of(ctx, slot));
       return;
     }
   }

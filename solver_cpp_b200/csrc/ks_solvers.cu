@@ -1217,8 +1217,9 @@ inline bool dia_pair_ok(const CsrDev &A, const CsrDev &T, long long n) {
 
 // A^T's diagonals as a view of A's copy: diagonal k (offset o) is A's
 // diagonal nd-1-k (offset -o) read o rows further on; masks are A^T's.
-inline DiaT<double> dview_mirror(const CsrDev &A, const CsrDev &T) {
-  DiaT<double> d = dview<double>(T);
+template <bool kC>
+inline DiaOf<double, kC> dview_mirror(const CsrDev &A, const CsrDev &T) {
+  DiaOf<double, kC> d = dview_of<kC, double>(T);
   const int nd = A.dia_nd;
   for (int k = 0; k < nd; k++) {
     d.vb[k] = A.dia_val + (long long)(nd - 1 - k) * A.dia_ds;
@@ -1236,14 +1237,15 @@ inline void launch_pair_n(ks_ctx *ctx, const CsrDev &A, const CsrDev &T, const d
   const long long wave = (long long)ctx->num_sms * spmv_dia_ctas_per_sm<1, NDG, double, GPtr<double>, EpiA>(ctx->device);
   ctx->next_class = kMv;
   const dim3 grid((unsigned)std::max<long long>(1, std::min(need, wave)));
-  auto run = [&](auto kern) {
-    launch_k(ctx, kern, grid, dim3(kThreads), 0, dview<double>(A), dview_mirror(A, T), GPtr<double>{p}, GPtr<double>{ps},
-             epi, stop, red_of(ctx, 0));
+  auto run = [&](auto c) {
+    constexpr bool kC = decltype(c)::value;
+    launch_k(ctx, spmv_dia_pair_kernel<NDG, GPtr<double>, Epi, kC>, grid, dim3(kThreads), 0, dview_of<kC, double>(A),
+             dview_mirror<kC>(A, T), GPtr<double>{p}, GPtr<double>{ps}, epi, stop, red_of(ctx, 0));
   };
   if (A.dia_cst && T.dia_cst)
-    run(spmv_dia_pair_kernel<NDG, GPtr<double>, Epi, true>);
+    run(std::true_type{});
   else
-    run(spmv_dia_pair_kernel<NDG, GPtr<double>, Epi, false>);
+    run(std::false_type{});
 }
 
 template <class EpiA, class Epi>

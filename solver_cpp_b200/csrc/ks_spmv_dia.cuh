@@ -19,7 +19,7 @@
 // reads 32 consecutive values of each diagonal and 32 consecutive entries of
 // x per diagonal (coalesced; x is shared by the diagonals through L1/L2).
 // Matrix data is read with the streaming hint, so the Krylov vectors keep
-// their place in L2. Where each diagonal's entries are one value (DiaT::cst:
+// their place in L2. Where each diagonal's entries are one value (DiaC:
 // Poisson, convection-diffusion with constant coefficients) the FP64 SpMV
 // takes it from the kernel's parameters: one mask byte per row instead of
 // 33 (symmetric half) or 57 bytes of a 7-point row, the same products and
@@ -46,12 +46,18 @@ struct DiaT {
   int cmin, cmax;  // columns that exist in x (a split rank's window: beyond its rows)
   int off[kMaxDiag];
   int quad;  // 1: the launcher enabled the quad path (spmv_dia_kernel; dia_quad_ok)
-  // 1 (FP64 values): every diagonal's entries are one value, cv[d] (a
-  // constant-coefficient stencil); the values are then not read at all, and
-  // the row masks alone say which terms a row has
-  int cst;
+};
+
+// With kC (CsrDev::dia_cst) every diagonal's entries are one value, cv[d] (a
+// constant-coefficient stencil): the values are then not read at all, and the row
+// masks alone say which terms a row has. A type of its own: as members of DiaT they
+// cost every launch of the other kernels 0.1 to 0.3 us of parameters.
+template <class MT>
+struct DiaC : DiaT<MT> {
   MT cv[kMaxDiag];
 };
+template <class MT, bool kC>
+using DiaOf = std::conditional_t<kC, DiaC<MT>, DiaT<MT>>;
 
 template <class MT>
 __device__ __forceinline__ MT ld_stream(const MT *p) {
@@ -193,11 +199,11 @@ __device__ __forceinline__ int dia_col(const DiaT<MT> &D, int i, int d) {
   return kIn ? c : min(max(c, D.cmin), D.cmax - 1);
 }
 
-// kC (FP64): every diagonal's entries are one value (DiaT::cst), taken from
+// kC (FP64): every diagonal's entries are one value (DiaC), taken from
 // the kernel's parameters; the loads left are x's, and the columns are clamped
 // only in warps whose rows reach past the ends.
 template <int NV, int NDG, class MT, class GX, class Epi, bool kC = false>
-__global__ void __launch_bounds__(kThreads) spmv_dia_kernel(DiaT<MT> D, GX gx0, GX gx1, Epi epi, Stop stop, Red red) {
+__global__ void __launch_bounds__(kThreads) spmv_dia_kernel(DiaOf<MT, kC> D, GX gx0, GX gx1, Epi epi, Stop stop, Red red) {
   using AT = typename Epi::acc_t;
   constexpr int ND = Epi::ND > 0 ? Epi::ND : 1;
   constexpr int K = NDG > 0 ? NDG : kMaxDiag;
@@ -287,7 +293,7 @@ __global__ void __launch_bounds__(kThreads) spmv_dia_kernel(DiaT<MT> D, GX gx0, 
 // masked out. epi.row(i, q, t, acc).
 template <int NDG, class GX, class Epi, bool kC>
 __global__ void __launch_bounds__(kThreads)
-    spmv_dia_pair_kernel(DiaT<double> DA, DiaT<double> DT, GX gx0, GX gx1, Epi epi, Stop stop, Red red) {
+    spmv_dia_pair_kernel(DiaOf<double, kC> DA, DiaOf<double, kC> DT, GX gx0, GX gx1, Epi epi, Stop stop, Red red) {
   constexpr int ND = Epi::ND > 0 ? Epi::ND : 1;
   double acc[ND];
 #pragma unroll
