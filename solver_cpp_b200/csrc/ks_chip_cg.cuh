@@ -841,14 +841,15 @@ inline bool chip_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShap
   long long rows = 0;
   if (A.dia_box) {
     // the tile with the least work: its rows, plus half a row for each of the
-    // halo's (fetched in the shadow of a reduction)
+    // halo's (fetched in the shadow of a reduction). Only heights that leave no more
+    // than G0 tiles in y and whose plane fits: the lines of a long box can be many
     s->nx = A.dia_off[5];
     s->ny = A.dia_off[6] / s->nx;
     s->nz = (int)(n / A.dia_off[6]);
     double best = 0.0;
-    for (int by = 1; by <= s->ny; by++) {
+    const int top = std::min(s->ny, kMaxRows / s->nx);
+    for (int by = (int)((s->ny + G0 - 1) / G0); by <= top; by++) {
       const int gy = (s->ny + by - 1) / by;
-      if (gy > G0) continue;
       const int bz = (int)((s->nz + G0 / gy - 1) / (G0 / gy));
       const double cost = (double)s->nx * ((double)by * bz + (by + bz));
       if ((long long)s->nx * by * bz > kMaxRows || (best > 0.0 && cost >= best)) continue;
@@ -959,15 +960,14 @@ inline bool tile_shape(const ks_ctx *ctx, const CsrDev &A, long long n, ChipShap
   s->ny = A.dia_off[6] / s->nx;
   s->nz = (int)(n / A.dia_off[6]);
   double best = 0.0;
-  for (int by = 1; by <= s->ny; by++) {
+  const int top = std::min(s->ny, kTileHaloZ * kTileHaloThreads / s->nx);  // as chip_shape
+  for (int by = (int)((s->ny + sms - 1) / sms); by <= top; by++) {
     const long long gy = (s->ny + by - 1) / by;
-    if (gy > sms) continue;
     const long long bz = (s->nz + sms / gy - 1) / (sms / gy);
     const long long elems = 2 + (long long)(s->nx + 1) * (by + 2) * (bz + 2);
     const long long halo = 2LL * s->nx * (by + bz), cols = ((long long)s->nx * by + kChipThreads - 1) / kChipThreads;
     const double cost = (double)(cols * ((bz + 7) / 8 * 8)) * kChipThreads + 0.5 * (double)halo;
-    if (cols * ((bz + 7) / 8 * 8) > kTileRows || (long long)s->nx * by > kTileHaloZ * kTileHaloThreads ||
-        s->nx * bz > kTileHaloY * kTileHaloThreads || elems > (1 << 20) ||
+    if (cols * ((bz + 7) / 8 * 8) > kTileRows || s->nx * bz > kTileHaloY * kTileHaloThreads || elems > (1 << 20) ||
         sizeof(double) * (size_t)elems + 2048 > (size_t)optin || (best > 0.0 && cost >= best))
       continue;
     best = cost;
