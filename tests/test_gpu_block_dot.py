@@ -58,3 +58,46 @@ def test_same_bits_with_fewer_vectors(ks, ctx, n, k, noalloc):
     for m in (1, 2, 8, 15, 16):
         if m < k:
             assert torch.equal(project(ks, ctx, V, w, m, noalloc), h[:m]), m
+
+
+CAPTURE = """
+import ctypes as C, sys
+import torch
+sys.path.insert(0, sys.argv[1])
+import solver_cpp_b200 as ks
+L = ks.lib()
+n, k = 1000003, 24
+V = torch.randn(k, n, device="cuda", dtype=torch.float64)
+w = torch.randn(n, device="cuda", dtype=torch.float64)
+h = torch.zeros(k, device="cuda", dtype=torch.float64)
+p = lambda t: C.c_void_p(t.data_ptr())
+s = torch.cuda.Stream()
+torch.cuda.synchronize()
+call = lambda n, k: L.ks_block_dot_noalloc(p(V), V.shape[1], k, p(w), n, p(h), C.c_void_p(s.cuda_stream))
+assert call(1000, 1) == 0  # the first call; a captured one may take the other kernel
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    assert call(n, k) == 0
+h.fill_(float("nan"))
+g.replay()
+torch.cuda.synchronize()
+bound = 1e-11 * V.norm(dim=1) * w.norm()
+assert bool(((h - V @ w).abs() <= bound).all())
+want = h.clone()
+assert call(n, k) == 0
+torch.cuda.synchronize()
+assert torch.equal(h, want)
+print("captured")
+"""
+
+
+def test_noalloc_under_capture_after_a_first_small_call():
+    """In a process of its own: the captured call is the first to take its kernel."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURE, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
