@@ -86,7 +86,8 @@ const char *ks_last_error(const ks_ctx *ctx);
 const char *ks_ctx_solve_kernel(const ks_ctx *ctx);
 int ks_abi_version(void);
 /* Limit of every bounded device wait of this context's kernels (the SpMV's
- * shared-memory staging barriers), in nanoseconds; ns <= 0 restores the
+ * shared-memory staging barriers, the grid-wide waits of the one-launch solves),
+ * in nanoseconds; ns <= 0 restores the
  * default of 2 s. A wait that runs out ends its kernel early with the
  * context's timeout flag set, and the call returns KS_TIMEOUT; the kernel
  * still drains its own copies in flight (bounded by the default limit), so
@@ -261,11 +262,11 @@ typedef struct {
                               FP32/BF16 inner CG: 0 auto, 1 x += alpha p
                               every iteration, 2 deferred through a ring of
                               32 directions (same x bit for bit)           */
-  int32_t cluster_solve;   /* CG, CR, BiCG on at most 32768 rows (one GPU): 0
-                              auto, the whole solve in one launch of one
-                              thread-block cluster where the device can hold
-                              it; 1 never (one kernel per step, as for larger
-                              systems)                                      */
+  int32_t cluster_solve;   /* CG, CR, BiCG (one GPU): 0 auto, the whole solve in
+                              one launch where the system fits, of one
+                              thread-block cluster on small systems, else of
+                              one CTA per SM (ks_ctx_solve_kernel); 1 never
+                              (one kernel per step, as for larger systems)  */
   int32_t inner_fast;      /* VP methods whose inner CG runs in FP32 / with
                               BF16 values on a one-GPU matrix with a diagonal
                               copy: 0 auto, the whole inner solve as one

@@ -32,7 +32,7 @@ ks_status check_device_error(ks_ctx *ctx) {
   KS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (flag) {
     KS_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    return set_error(ctx, KS_TIMEOUT, "a bounded wait on a shared-memory staging barrier ran out");
+    return set_error(ctx, KS_TIMEOUT, "a bounded device wait ran out");
   }
   return KS_OK;
 }
